@@ -2,9 +2,9 @@
 // Which tokens leave the ring in block j depends only on counts, and their write gates are
 // known before the block loop starts, so the per-block top-k (upstream memory_banks.py:486-552)
 // is hoisted out of the sequential chain: one warp per (state, block) stages the gates of the
-// evicted run in shared memory and lane 0 replays the host selection algorithm on them.
+// evicted run in shared memory and replays the host selection algorithm on them (topk_warp.cuh).
 #include "coda_common.cuh"
-#include "topk_order.h"
+#include "topk_warp.cuh"
 
 struct SelectParams {
   const float* gates; long long gates_bs;
@@ -13,13 +13,15 @@ struct SelectParams {
 };
 
 constexpr int SEL_WARPS = 4;
+constexpr size_t SEL_PER_TOKEN = sizeof(topk_order::Item<float>) + 2 * sizeof(uint16_t);     // queue entry + partition scratch
 
 __global__ void __launch_bounds__(SEL_WARPS * 32) select_kernel(SelectParams p, int cap) {
-  extern __shared__ unsigned char sel_sm[];
+  extern __shared__ __align__(16) unsigned char sel_sm[];
   typedef topk_order::Item<float> It;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   It* q = reinterpret_cast<It*>(sel_sm) + (size_t)warp * cap;
-  const long long prob = (long long)blockIdx.x * SEL_WARPS + warp;
+  uint16_t* scratch = reinterpret_cast<uint16_t*>(sel_sm + (size_t)nwarps * cap * sizeof(It)) + (size_t)warp * 2 * cap;
+  const long long prob = (long long)blockIdx.x * nwarps + warp;
   if (prob >= (long long)p.B * p.nblk) return;
   const int b = (int)(prob / p.nblk), j = (int)(prob % p.nblk);
   // counts before block j (memory_banks.py:459-466)
@@ -35,8 +37,7 @@ __global__ void __launch_bounds__(SEL_WARPS * 32) select_kernel(SelectParams p, 
   const float* g = p.gates + (long long)b * p.gates_bs + (seen - fill);   // first evicted token
   for (int i = lane; i < n_ev; i += 32) { q[i].v = g[i]; q[i].i = i; }
   __syncwarp();
-  if (lane == 0) topk_order::topk_queue<float, true>(q, n_ev, k, false);
-  __syncwarp();
+  topk_order::topk_queue_warp<float, true>(q, n_ev, k, false, scratch);
   for (int i = lane; i < k; i += 32) out[i] = q[i].i;
 }
 
@@ -55,13 +56,13 @@ extern "C" int coda_b200_select_candidates(const coda_layer_cfg* cfg, const floa
   CODA_REQUIRE(cand_stride >= (tmax < block ? tmax : block), CODA_ERR_ARG, "select_candidates: cand_stride too small");
   if (tmax == 0) return CODA_OK;
   const int cap = block;                                       // evict_len <= block
-  const size_t smem = (size_t)SEL_WARPS * cap * sizeof(topk_order::Item<float>);
-  CODA_REQUIRE(smem <= 200 * 1024, CODA_ERR_LIMIT, "select_candidates: block_size %d exceeds the limit of %d tokens",
-               block, (int)(200 * 1024 / (SEL_WARPS * sizeof(topk_order::Item<float>))));
+  CODA_REQUIRE(block <= 6400, CODA_ERR_LIMIT, "select_candidates: block_size %d exceeds the limit of %d tokens", block, 6400);
+  const int warps = SEL_WARPS * cap * SEL_PER_TOKEN <= 200 * 1024 ? SEL_WARPS : 1;
+  const size_t smem = (size_t)warps * cap * SEL_PER_TOKEN;
   if (smem > 48 * 1024) cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const long long nprob = (long long)cfg->B * p.nblk;
-  const int grid = (int)((nprob + SEL_WARPS - 1) / SEL_WARPS);
-  select_kernel<<<grid, SEL_WARPS * 32, smem, (cudaStream_t)stream>>>(p, cap);
+  const int grid = (int)((nprob + warps - 1) / warps);
+  select_kernel<<<grid, warps * 32, smem, (cudaStream_t)stream>>>(p, cap);
   CODA_CHECK_LAUNCH("select_candidates");
   return CODA_OK;
 }

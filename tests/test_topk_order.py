@@ -76,3 +76,33 @@ def test_known_answers():
     unused = lambda n: torch.full((n,), -(2 ** 62), dtype=torch.int64)  # noqa: E731
     assert _topk(unused(64), 8, False, True) == [44, 41, 42, 43, 46, 47, 40, 45]
     assert _topk(unused(32), 8, False, True) == [20, 23, 22, 21, 18, 17, 24, 19]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,fill0,L,block,Te,Ts", [
+    (256, 256, 1024, 256, 8, 64), (256, 0, 1000, 1024, 8, 64), (128, 100, 517, 97, 8, 64), (64, 64, 640, 64, 3, 2),
+    (16, 16, 4000, 4000, 8, 64), (32, 32, 6400, 6400, 8, 16), (8, 8, 48, 3, 8, 64), (64, 64, 192, 33, 33, 33)])
+def test_device_selection_equals_host_topk(W, fill0, L, block, Te, Ts):
+    """The warp's replay of the selection (partition passes by ballots and prefix counts) leaves the index lists of
+    torch.topk on the host, in their order, for distinct, tied and mixed gates; exact: indices."""
+    from coda_gqa_l_b200 import _lib as b
+    B, nblk = 8, (L + block - 1) // block
+    g = torch.Generator().manual_seed(W + L)
+    gates = torch.stack([_gates(i % 4, fill0 + L, g) for i in range(B)])
+    cfg = b.LayerCfg(B=B, H=2, Hkv=1, Dh=64, W=W, Me=4, Ms=4, dtype=b.CODA_F32, Te=Te, Ts=Ts)
+    dev = gates.cuda()
+    tmax = max(1, min(max(Te, Ts), block))
+    cand = torch.full((B, nblk, tmax), -1, dtype=torch.int32, device="cuda")
+    b.check(b.lib.coda_b200_select_candidates(C.byref(cfg), dev.data_ptr(), dev.stride(0), fill0, L, block, cand.data_ptr(), tmax,
+                                              torch.cuda.current_stream().cuda_stream), "select")
+    cand = cand.cpu()
+    for j in range(nblk):
+        seen = fill0 + j * block
+        fill, blk = min(seen, W), min(block, L - j * block)
+        n_ev = max(0, fill + blk - W)
+        k = max(min(Te, n_ev), min(Ts, n_ev))
+        if k == 0:
+            continue
+        for s in range(B):
+            ref = torch.topk(gates[s:s + 1, seen - fill:seen - fill + n_ev], k, dim=1, sorted=False)[1][0].tolist()
+            assert cand[s, j, :k].tolist() == ref, (s, j)
