@@ -89,167 +89,144 @@ __global__ void __launch_bounds__(256) prep_kernel(PrepParams p) {
   }
 }
 
-// 16-byte vectors of T <-> fp32
-template <typename T> struct Vec16;
-template <> struct Vec16<float> {
-  static constexpr int N = 4;
-  static __device__ __forceinline__ void ld(const float* p, float (&o)[4]) { const float4 v = *reinterpret_cast<const float4*>(p); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
-  static __device__ __forceinline__ void st(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
-};
-template <> struct Vec16<bf16> {
-  static constexpr int N = 8;
-  static __device__ __forceinline__ void ld(const bf16* p, float (&o)[8]) {
-    const uint4 v = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { o[2 * j] = __uint_as_float(w[j] << 16); o[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
-  }
-  static __device__ __forceinline__ void st(bf16* p, const float (&o)[8]) {
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { __nv_bfloat162 t = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]); w[j] = *reinterpret_cast<uint32_t*>(&t); }
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-};
-
 // Vectorised variant.  Work item = one 16-byte chunk of a head row (interleaved pairs) or the two chunks c and
 // c + Dh/2 that hold each other's RoPE partners (half-split pairs).  The noise query always rotates (even, odd)
 // neighbours of the ROTATED row (primitives.py:58-80), which lie inside one chunk, so an item is self-contained.
-template <typename T, typename A>
-__global__ void __launch_bounds__(320) prep_vec_kernel(PrepParams p) {
-  constexpr int N = Vec16<T>::N;
-  extern __shared__ float sm[];
+//
+// One CTA = a tile of `tt` consecutive positions of `nb` states: the states of a batch stand at the same positions, so
+// the cos / sin tables of the tile are evaluated once, all entries at the same time (an accurate sine is a chain of
+// some thousand cycles; one table per token is what bounded this kernel), and the tile's (token, item) pairs are dealt
+// out flat, so that a narrow layer's tokens, which have fewer items than a CTA has threads, leave none idle.
+// Bound: HBM (q and k in, q, k and the noise query out); what hides its latency is the number of resident threads, hence
+// the register limit and no per-thread state across items (tables from shared memory, the learned rotation from L1).
+// Measured, cold L2: 131072 tokens of a 512-wide layer 516 -> 123 us (3.8 TB/s), 131072 of a 576-wide 520 -> 118 us,
+// 16384 of a 4096-wide 102 -> 85 us, 8192 of an 8192-wide 86 -> 79 us (5.5 TB/s); three CTAs per SM with item state kept
+// in registers 98..130 us at 4096, five (32 registers, spilling) 97 us.
+template <typename T> struct Item;
+template <> struct Item<bf16> {             // tables as packed words; the arithmetic is one instruction per element pair
+  uint4 cv, sv;                             // half-split: cos / sin of angles 8c..8c+7; interleaved: pairs 4c..4c+3, each word duplicated
+  uint2 ca, sa, cb, sb;                     // learned rotation of the first / second chunk's four pairs
+  static __device__ __forceinline__ uint2 ld2(const bf16* p) { return *reinterpret_cast<const uint2*>(p); }
+  static __device__ __forceinline__ uint4 dup4(const uint2& w) { return make_uint4(bdup_lo(w.x), bdup_hi(w.x), bdup_lo(w.y), bdup_hi(w.y)); }
+  static __device__ __forceinline__ uint4 turn(const uint4& x, const uint4& c, const uint4& s) {
+    return make_uint4(brot(x.x, c.x, s.x), brot(x.y, c.y, s.y), brot(x.z, c.z, s.z), brot(x.w, c.w, s.w));
+  }
+  static __device__ __forceinline__ uint4 mix(const uint4& a, const uint4& c, const uint4& b, const uint4& s) {   // a c + b s
+    return make_uint4(badd2(bmul2(a.x, c.x), bmul2(b.x, s.x)), badd2(bmul2(a.y, c.y), bmul2(b.y, s.y)),
+                      badd2(bmul2(a.z, c.z), bmul2(b.z, s.z)), badd2(bmul2(a.w, c.w), bmul2(b.w, s.w)));
+  }
+  __device__ __forceinline__ void tables(const bf16* csb, const bf16* snb, bool inter, int c) {
+    if (inter) { cv = dup4(ld2(csb + 4 * c)); sv = dup4(ld2(snb + 4 * c)); }
+    else { cv = *reinterpret_cast<const uint4*>(csb + 8 * c); sv = *reinterpret_cast<const uint4*>(snb + 8 * c); }
+  }
+  __device__ __forceinline__ void theta(const bf16* cth, const bf16* sth, bool inter, int c, int half) {
+    ca = ld2(cth + 4 * c); sa = ld2(sth + 4 * c);
+    if (!inter) { cb = ld2(cth + (half >> 1) + 4 * c); sb = ld2(sth + (half >> 1) + 4 * c); }
+  }
+  __device__ __forceinline__ uint4 rope_pairs(const uint4& x) const { return turn(x, cv, sv); }
+  __device__ __forceinline__ void rope_halves(const uint4& x1, const uint4& x2, uint4& oa, uint4& ob) const {     // x1 c + (-x2) s ; x2 c + x1 s
+    oa = mix(x1, cv, make_uint4(bneg2(x2.x), bneg2(x2.y), bneg2(x2.z), bneg2(x2.w)), sv);
+    ob = mix(x2, cv, x1, sv);
+  }
+  __device__ __forceinline__ uint4 noise_a(const uint4& o) const { return turn(o, dup4(ca), dup4(sa)); }
+  __device__ __forceinline__ uint4 noise_b(const uint4& o) const { return turn(o, dup4(cb), dup4(sb)); }
+};
+template <> struct Item<float> {
+  float c[4], s[4];                         // half-split: angles 4c..4c+3; interleaved: pairs 2c, 2c+1 (first two)
+  float ta[2], ua[2], tb[2], ub[2];         // learned rotation cos / sin of the two pairs of the first / second chunk
+  static __device__ __forceinline__ float f(uint32_t w) { return __uint_as_float(w); }
+  static __device__ __forceinline__ uint32_t u(float v) { return __float_as_uint(v); }
+  static __device__ __forceinline__ uint4 turn(const uint4& x, float c0, float s0, float c1, float s1) {
+    return make_uint4(u(t_sub<float>(t_mul<float>(f(x.x), c0), t_mul<float>(f(x.y), s0))), u(t_add<float>(t_mul<float>(f(x.x), s0), t_mul<float>(f(x.y), c0))),
+                      u(t_sub<float>(t_mul<float>(f(x.z), c1), t_mul<float>(f(x.w), s1))), u(t_add<float>(t_mul<float>(f(x.z), s1), t_mul<float>(f(x.w), c1))));
+  }
+  __device__ __forceinline__ void tables(const float* cs, const float* sn, bool inter, int ch) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = inter ? 2 * ch + (e & 1) : 4 * ch + e;
+      c[e] = cs[i]; s[e] = sn[i];
+    }
+  }
+  __device__ __forceinline__ void theta(const float* cth, const float* sth, bool inter, int ch, int half) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      ta[e] = cth[2 * ch + e]; ua[e] = sth[2 * ch + e];
+      if (!inter) { tb[e] = cth[(half >> 1) + 2 * ch + e]; ub[e] = sth[(half >> 1) + 2 * ch + e]; }
+    }
+  }
+  __device__ __forceinline__ uint4 rope_pairs(const uint4& x) const { return turn(x, c[0], s[0], c[1], s[1]); }
+  __device__ __forceinline__ void rope_halves(const uint4& x1, const uint4& x2, uint4& oa, uint4& ob) const {
+    const uint32_t a[4] = {x1.x, x1.y, x1.z, x1.w}, b[4] = {x2.x, x2.y, x2.z, x2.w};
+    uint32_t p[4], q[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      p[e] = u(t_add<float>(t_mul<float>(f(a[e]), c[e]), t_mul<float>(-f(b[e]), s[e])));
+      q[e] = u(t_add<float>(t_mul<float>(f(b[e]), c[e]), t_mul<float>(f(a[e]), s[e])));
+    }
+    oa = make_uint4(p[0], p[1], p[2], p[3]); ob = make_uint4(q[0], q[1], q[2], q[3]);
+  }
+  __device__ __forceinline__ uint4 noise_a(const uint4& o) const { return turn(o, ta[0], ua[0], ta[1], ua[1]); }
+  __device__ __forceinline__ uint4 noise_b(const uint4& o) const { return turn(o, tb[0], ub[0], tb[1], ub[1]); }
+};
+
+template <typename T, typename A, bool INTER>
+__global__ void __launch_bounds__(320, 4) prep_vec_kernel(PrepParams p, int tt, int nb) {
+  constexpr int N = 16 / (int)sizeof(T);    // elements per 16-byte chunk
+  extern __shared__ __align__(16) unsigned char prep_sm[];
   const int half = p.Dh >> 1;
-  float* cs = sm;                 // [half] cos, rounded to T
-  float* sn = sm + half;          // [half] sin
-  bf16* csb = reinterpret_cast<bf16*>(sm + 2 * half);   // bf16 activations: the same tables as bf16, [half] cos | [half] sin
-  bf16* snb = csb + half;
-  constexpr bool PACKED = sizeof(T) == 2;
+  T* tab = reinterpret_cast<T*>(prep_sm);   // [tt][cos half | sin half], entries rounded to T
   const int tid = threadIdx.x, NT = blockDim.x;
-  const long long ntok = (long long)p.B * p.L;
-  const long long pos_base = ring_now(p.rp, p.W).pos;
-  const int per_head = p.interleaved ? p.Dh / N : half / N;       // items per head row
-  const int nq = p.H * per_head, nk = p.k ? p.Hkv * per_head : 0;
-  for (long long tok = blockIdx.x; tok < ntok; tok += gridDim.x) {
-    const int b = (int)(tok / p.L), t = (int)(tok % p.L);
-    const long long pos = pos_base + t;
-    __syncthreads();                                               // the previous token's table is no longer read
-    for (int i = tid; i < half; i += NT) {
-      float ta = El<A>::rnd((float)pos);
-      float inv = El<A>::rnd(p.inv_freq[i]);
-      float ang = El<A>::rnd(__fmul_rn(ta, inv));
-      cs[i] = El<T>::rnd(El<A>::rnd(cosf(ang)));
-      sn[i] = El<T>::rnd(El<A>::rnd(sinf(ang)));
-      if (PACKED) { csb[i] = __float2bfloat16_rn(cs[i]); snb[i] = __float2bfloat16_rn(sn[i]); }
-    }
-    __syncthreads();
-    T* qt = (T*)p.q + (long long)b * p.q_bs + (long long)t * p.q_rs;
-    T* kt = p.k ? (T*)p.k + (long long)b * p.k_bs + (long long)t * p.k_rs : nullptr;
-    T* qnt = (T*)p.qn + tok * (long long)(p.H * p.Dh);
-    for (int w = tid; w < nq + nk; w += NT) {
-      const bool isq = w < nq;
-      const int ww = isq ? w : w - nq;
-      const int h = ww / per_head, c = ww % per_head;
-      T* row = (isq ? qt : kt) + h * p.Dh;
-      const T* cth = (const T*)p.cos_t + h * half;
-      const T* sth = (const T*)p.sin_t + h * half;
-      if (PACKED) {
-        // eight elements per 16-byte vector, four words of two; the tables' entries come four at a time (8 bytes)
-        if (p.interleaved) {                // word j = pair i = 4c + j, rotated by the position's angle i
-          uint4 xv = *reinterpret_cast<const uint4*>(row + c * N);
-          const uint2 cw = *reinterpret_cast<const uint2*>(csb + 4 * c), sw = *reinterpret_cast<const uint2*>(snb + 4 * c);
-          uint4 ov;
-          ov.x = brot(xv.x, bdup_lo(cw.x), bdup_lo(sw.x)); ov.y = brot(xv.y, bdup_hi(cw.x), bdup_hi(sw.x));
-          ov.z = brot(xv.z, bdup_lo(cw.y), bdup_lo(sw.y)); ov.w = brot(xv.w, bdup_hi(cw.y), bdup_hi(sw.y));
-          *reinterpret_cast<uint4*>(row + c * N) = ov;
-          if (isq) {
-            const uint2 ct = *reinterpret_cast<const uint2*>(cth + 4 * c), st = *reinterpret_cast<const uint2*>(sth + 4 * c);
-            uint4 nv;
-            nv.x = brot(ov.x, bdup_lo(ct.x), bdup_lo(st.x)); nv.y = brot(ov.y, bdup_hi(ct.x), bdup_hi(st.x));
-            nv.z = brot(ov.z, bdup_lo(ct.y), bdup_lo(st.y)); nv.w = brot(ov.w, bdup_hi(ct.y), bdup_hi(st.y));
-            *reinterpret_cast<uint4*>(qnt + h * p.Dh + c * N) = nv;
-          }
-        } else {                            // x1 = elements 8c.., x2 = their partners half + 8c..; angles 8c..8c+7
-          const uint4 x1 = *reinterpret_cast<const uint4*>(row + c * N), x2 = *reinterpret_cast<const uint4*>(row + half + c * N);
-          const uint4 cv = *reinterpret_cast<const uint4*>(csb + c * N), sv = *reinterpret_cast<const uint4*>(snb + c * N);
-          uint4 oa, ob;                       // x1 c + (-x2) s ; x2 c + x1 s
-          oa.x = badd2(bmul2(x1.x, cv.x), bmul2(bneg2(x2.x), sv.x)); ob.x = badd2(bmul2(x2.x, cv.x), bmul2(x1.x, sv.x));
-          oa.y = badd2(bmul2(x1.y, cv.y), bmul2(bneg2(x2.y), sv.y)); ob.y = badd2(bmul2(x2.y, cv.y), bmul2(x1.y, sv.y));
-          oa.z = badd2(bmul2(x1.z, cv.z), bmul2(bneg2(x2.z), sv.z)); ob.z = badd2(bmul2(x2.z, cv.z), bmul2(x1.z, sv.z));
-          oa.w = badd2(bmul2(x1.w, cv.w), bmul2(bneg2(x2.w), sv.w)); ob.w = badd2(bmul2(x2.w, cv.w), bmul2(x1.w, sv.w));
-          *reinterpret_cast<uint4*>(row + c * N) = oa;
-          *reinterpret_cast<uint4*>(row + half + c * N) = ob;
-          if (isq) {                        // (even, odd) neighbours of the rotated row: pairs 4c.. and half/2 + 4c..
-            const uint2 cta = *reinterpret_cast<const uint2*>(cth + 4 * c), sta = *reinterpret_cast<const uint2*>(sth + 4 * c);
-            const uint2 ctb = *reinterpret_cast<const uint2*>(cth + (half >> 1) + 4 * c), stb = *reinterpret_cast<const uint2*>(sth + (half >> 1) + 4 * c);
-            uint4 na, nb;
-            na.x = brot(oa.x, bdup_lo(cta.x), bdup_lo(sta.x)); na.y = brot(oa.y, bdup_hi(cta.x), bdup_hi(sta.x));
-            na.z = brot(oa.z, bdup_lo(cta.y), bdup_lo(sta.y)); na.w = brot(oa.w, bdup_hi(cta.y), bdup_hi(sta.y));
-            nb.x = brot(ob.x, bdup_lo(ctb.x), bdup_lo(stb.x)); nb.y = brot(ob.y, bdup_hi(ctb.x), bdup_hi(stb.x));
-            nb.z = brot(ob.z, bdup_lo(ctb.y), bdup_lo(stb.y)); nb.w = brot(ob.w, bdup_hi(ctb.y), bdup_hi(stb.y));
-            *reinterpret_cast<uint4*>(qnt + h * p.Dh + c * N) = na;
-            *reinterpret_cast<uint4*>(qnt + h * p.Dh + half + c * N) = nb;
-          }
-        }
-      } else if (p.interleaved) {                  // primitives.py:99-106: pairs (2i, 2i+1) share cos/sin i
-        float x[N], o[N];
-        Vec16<T>::ld(row + c * N, x);
-#pragma unroll
-        for (int e = 0; e < N; e += 2) {
-          const int i = (c * N + e) >> 1;
-          const float cc = cs[i], ss = sn[i];
-          o[e] = t_sub<T>(t_mul<T>(x[e], cc), t_mul<T>(x[e + 1], ss));
-          o[e + 1] = t_add<T>(t_mul<T>(x[e], ss), t_mul<T>(x[e + 1], cc));
-        }
-        Vec16<T>::st(row + c * N, o);
-        if (isq) {
-          float n[N];
-#pragma unroll
-          for (int e = 0; e < N; e += 2) {
-            const int i = (c * N + e) >> 1;
-            const float ct = El<T>::ld(cth + i), st = El<T>::ld(sth + i);
-            n[e] = t_sub<T>(t_mul<T>(o[e], ct), t_mul<T>(o[e + 1], st));
-            n[e + 1] = t_add<T>(t_mul<T>(o[e], st), t_mul<T>(o[e + 1], ct));
-          }
-          Vec16<T>::st(qnt + h * p.Dh + c * N, n);
-        }
-      } else {                              // primitives.py:108-113: x*cos_full + rotate_half(x)*sin_full
-        float x1[N], x2[N], oa[N], ob[N];
-        Vec16<T>::ld(row + c * N, x1);
-        Vec16<T>::ld(row + half + c * N, x2);
-#pragma unroll
-        for (int e = 0; e < N; ++e) {
-          const float cc = cs[c * N + e], ss = sn[c * N + e];
-          oa[e] = t_add<T>(t_mul<T>(x1[e], cc), t_mul<T>(-x2[e], ss));
-          ob[e] = t_add<T>(t_mul<T>(x2[e], cc), t_mul<T>(x1[e], ss));
-        }
-        Vec16<T>::st(row + c * N, oa);
-        Vec16<T>::st(row + half + c * N, ob);
-        if (isq) {
-          float na[N], nb[N];
-#pragma unroll
-          for (int e = 0; e < N; e += 2) {
-            const int ia = (c * N + e) >> 1, ib = (half + c * N + e) >> 1;
-            const float cta = El<T>::ld(cth + ia), sta = El<T>::ld(sth + ia);
-            const float ctb = El<T>::ld(cth + ib), stb = El<T>::ld(sth + ib);
-            na[e] = t_sub<T>(t_mul<T>(oa[e], cta), t_mul<T>(oa[e + 1], sta));
-            na[e + 1] = t_add<T>(t_mul<T>(oa[e], sta), t_mul<T>(oa[e + 1], cta));
-            nb[e] = t_sub<T>(t_mul<T>(ob[e], ctb), t_mul<T>(ob[e + 1], stb));
-            nb[e + 1] = t_add<T>(t_mul<T>(ob[e], stb), t_mul<T>(ob[e + 1], ctb));
-          }
-          Vec16<T>::st(qnt + h * p.Dh + c * N, na);
-          Vec16<T>::st(qnt + h * p.Dh + half + c * N, nb);
-        }
-      }
-    }
-    for (int h = tid; h < p.H; h += NT) {
-      const float z = El<T>::ld((const T*)p.lam_logit + (long long)b * p.lam_bs + (long long)t * p.lam_rs + h);
-      p.lam[tok * p.H + h] = t_sigmoid<T>(z);
-    }
-    if (tid == 0 && p.gate != nullptr) {
+  const int t0 = blockIdx.x * tt, tn = min(tt, p.L - t0), b0 = blockIdx.y * nb, bn = min(nb, p.B - b0);
+  constexpr int CH = INTER ? 1 : 2;         // chunks of an item
+  const int per_head = p.Dh / (N * CH);     // items per head row
+  const int nq = p.H * per_head, nit = nq + (p.k ? p.Hkv * per_head : 0), ntok = tn * bn;
+  const long long pos = ring_now(p.rp, p.W).pos + t0;
+  for (int i = tid; i < tn * half; i += NT) {
+    // upstream primitives.py:51-54: t = arange(dtype=inv_freq.dtype); freqs = t (x) inv_freq; cos().to(dtype)
+    const int ti = i / half, j = i - ti * half;
+    float ta = El<A>::rnd((float)(pos + ti));
+    float inv = El<A>::rnd(p.inv_freq[j]);
+    float ang = El<A>::rnd(__fmul_rn(ta, inv));
+    float cc, ss; sincos_call(ang, &ss, &cc);
+    El<T>::st(tab + ti * p.Dh + j, El<T>::rnd(El<A>::rnd(cc)));
+    El<T>::st(tab + ti * p.Dh + half + j, El<T>::rnd(El<A>::rnd(ss)));
+  }
+  // lambda and gate sigmoids of the tile's tokens: item (token, head), the head after the last one being the gate
+  for (int i = tid; i < ntok * (p.H + 1); i += NT) {
+    const int u = i / (p.H + 1), hh = i - u * (p.H + 1), tq = u / bn, bq = b0 + u - tq * bn, ta = t0 + tq;
+    const long long tok = (long long)bq * p.L + ta;
+    if (hh < p.H) {
+      p.lam[tok * p.H + hh] = t_sigmoid<T>(El<T>::ld((const T*)p.lam_logit + (long long)bq * p.lam_bs + (long long)ta * p.lam_rs + hh));
+    } else if (p.gate != nullptr) {
       float g = 1.0f;                       // write_policy "none": attention.py:407-408
-      if (p.gated) g = t_sigmoid<T>(El<T>::ld((const T*)p.gate_logit + (long long)b * p.gate_bs + (long long)t * p.gate_rs));
+      if (p.gated) g = t_sigmoid<T>(El<T>::ld((const T*)p.gate_logit + (long long)bq * p.gate_bs + (long long)ta * p.gate_rs));
       p.gate[tok] = g;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < ntok * nit; i += NT) {
+    const int u = i / nit, w = i - u * nit, t = u / bn, b = b0 + u - t * bn;
+    const bool isq = w < nq;
+    const int ww = isq ? w : w - nq, h = ww / per_head, c = ww - h * per_head;
+    T* row = (isq ? (T*)p.q : (T*)p.k) + (long long)b * (isq ? p.q_bs : p.k_bs) + (long long)(t0 + t) * (isq ? p.q_rs : p.k_rs) + h * p.Dh + c * N;
+    T* nrow = (T*)p.qn + ((long long)b * p.L + t0 + t) * (long long)(p.H * p.Dh) + h * p.Dh + c * N;
+    Item<T> it;
+    if (INTER) {                            // primitives.py:99-106: pairs (2i, 2i+1) share cos/sin i
+      const uint4 x = *reinterpret_cast<const uint4*>(row);
+      if (isq) it.theta((const T*)p.cos_t + h * half, (const T*)p.sin_t + h * half, INTER, c, half);
+      it.tables(tab + t * p.Dh, tab + t * p.Dh + half, INTER, c);
+      const uint4 o = it.rope_pairs(x);
+      *reinterpret_cast<uint4*>(row) = o;
+      if (isq) *reinterpret_cast<uint4*>(nrow) = it.noise_a(o);
+    } else {                                // primitives.py:108-113: x*cos_full + rotate_half(x)*sin_full
+      const uint4 x1 = *reinterpret_cast<const uint4*>(row), x2 = *reinterpret_cast<const uint4*>(row + half);
+      if (isq) it.theta((const T*)p.cos_t + h * half, (const T*)p.sin_t + h * half, INTER, c, half);
+      it.tables(tab + t * p.Dh, tab + t * p.Dh + half, INTER, c);
+      uint4 oa, ob;
+      it.rope_halves(x1, x2, oa, ob);
+      *reinterpret_cast<uint4*>(row) = oa;
+      *reinterpret_cast<uint4*>(row + half) = ob;
+      if (isq) { *reinterpret_cast<uint4*>(nrow) = it.noise_a(oa); *reinterpret_cast<uint4*>(nrow + half) = it.noise_b(ob); }
     }
   }
 }
@@ -283,8 +260,24 @@ extern "C" int coda_b200_prep(const coda_layer_cfg* cfg, int32_t L, coda_ring_po
   const int vn = cfg->dtype == CODA_F32 ? 4 : 8;
   const bool vec = ((cfg->rope_interleaved ? cfg->Dh : cfg->Dh / 2) % vn) == 0 && ((uintptr_t)q | (uintptr_t)q_noise) % 16 == 0 &&
                    (q_bs | q_rs) % vn == 0 && (k == nullptr || ((uintptr_t)k % 16 == 0 && (k_bs | k_rs) % vn == 0));
+  // Tile of a CTA: positions so that the tables' entries keep the threads busy once, then states; no larger than leaves
+  // two waves of four CTAs per SM.
+  const long long share = ntok / (148LL * 8) > 1 ? ntok / (148LL * PREP_S) : 1;
+  int tt = 320 / (cfg->Dh / 2);
+  tt = tt < 1 ? 1 : (tt > 8 ? 8 : tt);
+  if (tt > share) tt = (int)share;
+  if (tt > L) tt = L;
+  long long nb = share / tt;
+  nb = nb < 1 ? 1 : (nb > cfg->B ? cfg->B : nb);
+  while ((cfg->B + nb - 1) / nb > 65535) ++nb;
 #define LAUNCH(T, A) do { \
-    if (vec) { prep_vec_kernel<T, A><<<grid, 320, sizeof(float) * (size_t)cfg->Dh + 2 * sizeof(bf16) * (size_t)(cfg->Dh / 2), s>>>(p); break; } \
+    if (vec) { \
+      const dim3 vgrid((unsigned)((L + tt - 1) / tt), (unsigned)((cfg->B + nb - 1) / nb)); \
+      const size_t vsmem = sizeof(T) * (size_t)cfg->Dh * tt; \
+      if (cfg->rope_interleaved) prep_vec_kernel<T, A, true><<<vgrid, 320, vsmem, s>>>(p, tt, (int)nb); \
+      else prep_vec_kernel<T, A, false><<<vgrid, 320, vsmem, s>>>(p, tt, (int)nb); \
+      break; \
+    } \
     if (smem > 48 * 1024) cudaFuncSetAttribute(prep_kernel<T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     prep_kernel<T, A><<<grid, 256, smem, s>>>(p); } while (0)
   if (cfg->dtype == CODA_F32) {
