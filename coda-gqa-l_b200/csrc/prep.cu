@@ -262,7 +262,7 @@ extern "C" int coda_b200_prep(const coda_layer_cfg* cfg, int32_t L, coda_ring_po
                    (q_bs | q_rs) % vn == 0 && (k == nullptr || ((uintptr_t)k % 16 == 0 && (k_bs | k_rs) % vn == 0));
   // Tile of a CTA: positions so that the tables' entries keep the threads busy once, then states; no larger than leaves
   // two waves of four CTAs per SM.
-  const long long share = ntok / (148LL * 8) > 1 ? ntok / (148LL * PREP_S) : 1;
+  const long long share = ntok / (148LL * 8) > 1 ? ntok / (148LL * 8) : 1;
   int tt = 320 / (cfg->Dh / 2);
   tt = tt < 1 ? 1 : (tt > 8 ? 8 : tt);
   if (tt > share) tt = (int)share;
