@@ -1,35 +1,34 @@
 // Chunked-prefill differential attention on the 5th-generation tensor cores (tcgen05 + TMEM), bf16.
 //
-// One CTA = one (state, query head, 128-row query tile) and BOTH streams: signal Q and theta-rotated noise Q
-// share every K/V tile.  Keys are the layer's Lbuf slots (masked by `allowed`) followed by the block's own
-// tokens (causal).  Per 128-key tile and stream:
-//     S = Q . K^T          tcgen05.mma  M=128 N=128 K=Dh   A, B from shared memory, S in TMEM
+// One CTA = one (state, query head, 64-row query tile) and BOTH streams, stacked as the 128 rows of every MMA: rows
+// 0..63 carry the signal Q, rows 64..127 the theta-rotated noise Q of the same tokens, so the two streams share every
+// K/V tile.  Keys are the layer's Lbuf slots (masked by `allowed`; 64-key tiles without a visible slot are skipped)
+// followed by the block's own tokens (causal).  Per 64-key tile:
+//     S = Q . K^T          tcgen05.mma  M=128 N=64 K=Dh    A, B from shared memory, S in TMEM
 //     P = exp2(S - m)      softmax warps: tcgen05.ld, lazy-rescaled online softmax, bf16 P written back over S
-//     O += P . V           tcgen05.mma  M=128 N=Dh  K=128  A = P straight from TMEM, B = V from shared memory
-// Warp roles: warps 0-3 = softmax / correction / epilogue of the signal stream, warps 4-7 = the same for the
-// noise stream (one thread per query row, the whole row of S in registers: setmaxnreg gives these two
-// warpgroups 208 registers), warp 8 = TMA producer (cp.async.bulk.tensor, 128-byte swizzle, 2-stage ring of
-// 128-key K/V tiles), warp 9 = MMA issuer and TMEM owner.  The two streams ping-pong on the
-// tensor core: while one stream is in softmax the other's P.V and next Q.K^T run.  Keeping P in TMEM halves
-// the shared-memory operand traffic of P.V and N=128 tiles keep Q.K^T at the operand-bandwidth limit.
-// TMEM map (512 columns): S_sig 0..127 (P_sig aliases 0..63), S_noise 128..255, O_sig 256.., O_noise 256+Dh..
-// Epilogue: O/l per stream, sig - lambda*noise, optional RMSNorm over Dh, bf16 rows written in the (B, L, H*Dh)
-// layout the output projection reads.  All mbarrier waits are bounded (status word, no hang, TMEM is freed).
+//     O += P . V           tcgen05.mma  M=128 N=Dh K=64    A = P straight from TMEM, B = V from shared memory
+// Warp roles: warps 0-3 = softmax / correction / epilogue (one thread per row), warp 4 = TMA producer (128-byte
+// swizzle, K and V on rings of their own), warp 5 = MMA issuer and TMEM owner.
+// What bounds it: the softmax warps' issue slots and special-function work.  Everything else is arranged so that they
+// do not wait.  S is double-buffered (S0, S1: 128 TMEM columns; with O at most 256), so Q.K^T of the next tile is
+// complete before the softmax of the present one ends, and half the tensor memory per CTA lets two CTAs share an SM:
+// one CTA's start-up and epilogue (a third of a CTA's life) run under the other's tiles.
+// Measured per block (two streams of 128 rows in one CTA per SM, 128-key tiles, before): 64 states x 8 heads x 256 queries
+// over 384 slots, Dh 64: 109 -> 94 us; 512 x 9 x 128 over 192, Dh 64: 352 -> 258 us; 32 x 32 x 128 over 384, Dh 128:
+// 115 -> 104 us; 8 x 64 x 256 over 768, Dh 128: 179 -> 165 us; 1 x 32 x 1000 over an empty state, Dh 128: 59 -> 42 us.
+// All mbarrier waits are bounded (status word, no hang, TMEM is freed).
 #include "coda_common.cuh"
 #include "tma_utils.cuh"
 #include "tensor_maps.h"
 
 namespace {
 
-constexpr int PF_BM = 128;       // query rows per CTA
-constexpr int PF_BN = 128;       // keys per tile
-// Register split after launch (setmaxnreg): the two softmax warpgroups grow, the third warpgroup shrinks.  A
-// warpgroup that asks for more than the CTA's pool (threads x registers at launch) can give waits forever, so the
-// launcher checks the sum against the kernel's compiled register count and refuses to launch otherwise.
-constexpr int PF_REGS_SOFTMAX = 208, PF_REGS_AUX = 72;
-constexpr int PF_REGS_TOTAL = 256 * PF_REGS_SOFTMAX + 128 * PF_REGS_AUX;
-constexpr int PF_THREADS = 384;  // warps 0-3 / 4-7: softmax of the signal / noise stream, 8: TMA, 9: MMA issuer, 10-11 idle
-constexpr int PF_STAGES = 2;     // K/V tiles in flight
+constexpr int PF_BM = 64;        // query rows per CTA (each present twice: signal and noise)
+constexpr int PF_BN = 64;        // keys per tile
+constexpr int PF_M = 128;        // MMA rows
+constexpr int PF_THREADS = 192;  // warps 0-3: softmax, 4: TMA, 5: MMA issuer
+constexpr int PF_TMEM_COLS = 256;
+constexpr int pf_stages(int dh) { return dh == 128 ? 2 : 3; }   // K tiles (and V tiles) in flight; two CTAs fit an SM
 constexpr float PF_RESCALE_GAP = 8.0f;   // log2 units the running max may lag before O is rescaled
 
 struct PrefillParams {
@@ -82,15 +81,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
                  "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                : "r"(taddr));
 }
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-               "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                 "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                 "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-               : "memory");
-}
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
@@ -116,7 +106,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes,
 // Instruction descriptor: fp32 accumulate, bf16 x bf16, M = 128, N = n, A K-major, B K-major or MN-major.
 __device__ __forceinline__ constexpr uint32_t instr_desc(int n, bool b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(PF_BM >> 4) << 24);
+         ((uint32_t)(PF_M >> 4) << 24);
 }
 // 2^x for x <= 0 on the special-function unit (one MUFU op).
 __device__ __forceinline__ float ex2_mufu(float x) {
@@ -171,208 +161,209 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-__device__ __forceinline__ void bar_softmax_all() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void bar_softmax_all() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
 template <int DH>
-__global__ void __launch_bounds__(PF_THREADS, 1)
+__global__ void __launch_bounds__(PF_THREADS, 2)
 prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap qnmap,
                       const __grid_constant__ CUtensorMap kpmap, const __grid_constant__ CUtensorMap vpmap,
                       const __grid_constant__ CUtensorMap kbmap, const __grid_constant__ CUtensorMap vbmap,
                       PrefillParams p) {
+  constexpr int STAGES = pf_stages(DH);
   constexpr int HALVES = DH / 64;                 // 64-element (128-byte) column groups per row
-  constexpr int Q_HALF = PF_BM * 128;             // bytes of one Q half tile
+  constexpr int Q_HALF = PF_M * 128;              // bytes of one column group of the stacked Q tile
   constexpr int Q_BYTES = HALVES * Q_HALF;
   constexpr int KV_HALF = PF_BN * 128;
   constexpr int KV_BYTES = HALVES * KV_HALF;      // one K (or V) tile
   constexpr int KSTEPS_QK = DH / 16;
   constexpr int KSTEPS_PV = PF_BN / 16;
-  constexpr uint32_t TM_SN = 128, TM_OS = 256, TM_ON = 256 + DH;   // TMEM column offsets (S_sig at 0)
+  constexpr uint32_t TM_O = 2 * PF_BN;            // TMEM columns: S0 at 0, S1 at 64, O at 128
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  unsigned char* sQs = smem;
-  unsigned char* sQn = sQs + Q_BYTES;
-  unsigned char* sK = sQn + Q_BYTES;               // [PF_STAGES][KV_BYTES]
-  unsigned char* sV = sK + PF_STAGES * KV_BYTES;   // [PF_STAGES][KV_BYTES]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + PF_STAGES * KV_BYTES);
+  unsigned char* sQ = smem;                        // [HALVES][128 rows][128 B]: rows 0..63 signal, 64..127 noise
+  unsigned char* sK = sQ + Q_BYTES;                // [STAGES][KV_BYTES]
+  unsigned char* sV = sK + STAGES * KV_BYTES;      // [STAGES][KV_BYTES]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + STAGES * KV_BYTES);
   uint64_t* q_full = bars;                          // 1
-  uint64_t* kv_full = bars + 1;                     // PF_STAGES
-  uint64_t* kv_empty = kv_full + PF_STAGES;         // PF_STAGES
-  uint64_t* s_full = kv_empty + PF_STAGES;          // [stream]
-  uint64_t* p_full = s_full + 2;                    // [stream]
-  uint64_t* pv_done = p_full + 2;                   // [stream]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
-  uint32_t* sMask = tmem_slot + 2;                  // visibility bits of the prefix slots, 32 per word
+  uint64_t* pv_done = bars + 1;                     // [buffer]
+  uint64_t* s_full = bars + 3;                      // [buffer]
+  uint64_t* p_full = bars + 5;                      // [buffer]
+  uint64_t* k_full = bars + 7;                      // [stage]
+  uint64_t* k_empty = k_full + STAGES;
+  uint64_t* v_full = k_empty + STAGES;
+  uint64_t* v_empty = v_full + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + STAGES);   // TMEM base, then the number of prefix tiles
+  uint32_t* sMask = tmem_slot + 2;                  // [NP][2] visibility bits of the n-th tile that is read
+  const int NP = (p.Lbuf + PF_BN - 1) / PF_BN;      // prefix tiles
+  unsigned short* sTile = reinterpret_cast<unsigned short*>(sMask + 2 * NP);   // [NP] which tile that is
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = blockIdx.x * PF_BM, h = blockIdx.y, b = blockIdx.z;
   const int hk = h / (p.H / p.Hkv);
-  const int NP = (p.Lbuf + PF_BN - 1) / PF_BN;                                   // prefix tiles
-  const int last_row = min(r0 + PF_BM, p.blk) - 1;
-  const int NB = last_row / PF_BN + 1;                                            // block tiles (causal limit)
-  const int NT = NP + NB;
 
   __shared__ int s_abort;                          // set by the first bounded wait of this CTA that expires
   int* const abortw = &s_abort;
-  if (tid == 0) {
-    s_abort = 0;
-    tma::mbar_init(q_full, 1);
-    for (int i = 0; i < PF_STAGES; ++i) { tma::mbar_init(&kv_full[i], 1); tma::mbar_init(&kv_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], 4); tma::mbar_init(&pv_done[i], 1); }
-    tma::fence_barrier_init();
-  }
-  if (warp == 9) {                                   // TMEM: all 512 columns, owned by the MMA warp
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    tc_fence_before();
-  }
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-
-  // Registers follow the roles, per warpgroup: a softmax thread keeps a whole row of S (128 values) in registers.
-  if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PF_REGS_AUX));
-  if (warp == 8) {
-    // =========================== TMA producer ===========================
+  if (warp == 4) {
     if (lane == 0) {
-      tma::mbar_expect_tx(q_full, 2 * Q_BYTES);
+      s_abort = 0;
+      tma::mbar_init(q_full, 1);
+      for (int i = 0; i < 2; ++i) { tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], 4); tma::mbar_init(&pv_done[i], 1); }
+      for (int i = 0; i < STAGES; ++i) {
+        tma::mbar_init(&k_full[i], 1); tma::mbar_init(&k_empty[i], 1);
+        tma::mbar_init(&v_full[i], 1); tma::mbar_init(&v_empty[i], 1);
+      }
+      tma::fence_barrier_init();
+      tma::mbar_expect_tx(q_full, Q_BYTES);         // (the barriers are this thread's own so far: Q may leave at once)
 #pragma unroll
       for (int hf = 0; hf < HALVES; ++hf) {
-        tma_load_4d(sQs + hf * Q_HALF, &qmap, q_full, hf * 64, h, p.t0 + r0, b);
-        tma_load_4d(sQn + hf * Q_HALF, &qnmap, q_full, hf * 64, h, p.t0 + r0, b);
+        tma_load_4d(sQ + hf * Q_HALF, &qmap, q_full, hf * 64, h, p.t0 + r0, b);
+        tma_load_4d(sQ + hf * Q_HALF + PF_BM * 128, &qnmap, q_full, hf * 64, h, p.t0 + r0, b);
       }
-      for (int j = 0; j < NT; ++j) {
-        const int st = j % PF_STAGES;
-        if (j >= PF_STAGES) tma::mbar_wait(&kv_empty[st], ((j / PF_STAGES) - 1) & 1, p.status, 11, abortw);
-        tma::mbar_expect_tx(&kv_full[st], 2 * KV_BYTES);
-        unsigned char* kd = sK + st * KV_BYTES;
-        unsigned char* vd = sV + st * KV_BYTES;
+    }
+  } else if (warp == 5) {                            // TMEM: half of the SM's columns, owned by the MMA warp
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(PF_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    tc_fence_before();
+  } else if (warp == 0) {                            // visibility of the prefix slots; tiles with no visible slot drop out
+    const uint8_t* al = p.allowed + (long long)b * p.Lbuf;
+    int nv = 0;
+    for (int j0 = 0; j0 < NP; j0 += 4) {
+      bool vis[8];
 #pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) {
-          if (j < NP) {
-            tma_load_3d(kd + hf * KV_HALF, &kpmap, &kv_full[st], hf * 64, j * PF_BN, b * p.Hkv + hk);
-            tma_load_3d(vd + hf * KV_HALF, &vpmap, &kv_full[st], hf * 64, j * PF_BN, b * p.Hkv + hk);
-          } else {
-            tma_load_4d(kd + hf * KV_HALF, &kbmap, &kv_full[st], hf * 64, hk, p.t0 + (j - NP) * PF_BN, b);
-            tma_load_4d(vd + hf * KV_HALF, &vbmap, &kv_full[st], hf * 64, hk, p.t0 + (j - NP) * PF_BN, b);
-          }
+      for (int i = 0; i < 8; ++i) {
+        const int c = j0 * PF_BN + i * 32 + lane;
+        vis[i] = c < p.Lbuf && (!p.mask_unused || al[c] != 0);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned lo = __ballot_sync(0xffffffffu, vis[2 * i]), hi = __ballot_sync(0xffffffffu, vis[2 * i + 1]);
+        if ((lo | hi) != 0u) {
+          if (lane == 0) { sTile[nv] = (unsigned short)(j0 + i); sMask[2 * nv] = lo; sMask[2 * nv + 1] = hi; }
+          ++nv;
         }
       }
     }
-  } else if (warp == 9) {
+    if (lane == 0) tmem_slot[1] = (uint32_t)nv;
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot[0];
+  const int NV = (int)tmem_slot[1];                  // prefix tiles that are read
+  const int NT = NV + r0 / PF_BN + 1;                // ... and the block tiles up to the diagonal
+
+  if (warp == 4) {
+    // =========================== TMA producer ===========================
+    if (lane == 0) {
+      auto load_tile = [&](int it, const CUtensorMap* pm, const CUtensorMap* bm, unsigned char* ring, uint64_t* full, uint64_t* empty, int code) {
+        const int st = it % STAGES;
+        if (it >= STAGES) tma::mbar_wait(&empty[st], ((it / STAGES) - 1) & 1, p.status, code, abortw);
+        tma::mbar_expect_tx(&full[st], KV_BYTES);
+        unsigned char* dst = ring + st * KV_BYTES;
+#pragma unroll
+        for (int hf = 0; hf < HALVES; ++hf) {
+          if (it < NV) tma_load_3d(dst + hf * KV_HALF, pm, &full[st], hf * 64, (int)sTile[it] * PF_BN, b * p.Hkv + hk);
+          else tma_load_4d(dst + hf * KV_HALF, bm, &full[st], hf * 64, hk, p.t0 + (it - NV) * PF_BN, b);
+        }
+      };
+      // K runs one tile ahead of V: its stage is free as soon as Q.K^T is done, long before P.V
+      load_tile(0, &kpmap, &kbmap, sK, k_full, k_empty, 11);
+      for (int it = 0; it < NT; ++it) {
+        if (it + 1 < NT) load_tile(it + 1, &kpmap, &kbmap, sK, k_full, k_empty, 11);
+        load_tile(it, &vpmap, &vbmap, sV, v_full, v_empty, 15);
+      }
+    }
+  } else if (warp == 5) {
     // =========================== MMA issuer ===========================
     if (lane == 0) {
       constexpr uint32_t IDESC_QK = instr_desc(PF_BN, false);
       constexpr uint32_t IDESC_PV = instr_desc(DH, true);
-      // S_s = Q_s . K_j^T  (the stream's S columns are free: its previous P.V, which read P from them, was
-      // issued earlier by this same thread and the tensor pipe executes in order)
-      auto issue_qk = [&](int j, int s) {
-        const uint32_t kbase = smem_u32(sK + (j % PF_STAGES) * KV_BYTES);
-        const uint32_t qbase = smem_u32(s ? sQn : sQs);
-        const uint32_t dcol = tmem + (s ? TM_SN : 0u);
+      const uint32_t qbase = smem_u32(sQ);
+      // S = Q . K^T into buffer it & 1 (free: the P.V two tiles back, which read P from it, was issued earlier by
+      // this same thread and the tensor pipe executes in order)
+      auto issue_qk = [&](int it) {
+        const int st = it % STAGES;
+        tma::mbar_wait(&k_full[st], (it / STAGES) & 1, p.status, 14, abortw);
+        tc_fence_after();
+        const uint32_t kbase = smem_u32(sK + st * KV_BYTES);
+        const uint32_t dcol = tmem + (uint32_t)(it & 1) * PF_BN;
 #pragma unroll
         for (int kk = 0; kk < KSTEPS_QK; ++kk) {
           const uint64_t ad = smem_desc(qbase + (kk >> 2) * Q_HALF + (kk & 3) * 32, 16, 1024);
           const uint64_t bd = smem_desc(kbase + (kk >> 2) * KV_HALF + (kk & 3) * 32, 16, 1024);
           tc_mma(dcol, ad, bd, IDESC_QK, kk > 0 ? 1u : 0u);
         }
-        tc_commit(&s_full[s]);
+        tc_commit(&s_full[it & 1]);
+        tc_commit(&k_empty[st]);
       };
       tma::mbar_wait(q_full, 0, p.status, 13, abortw);
-      tma::mbar_wait(&kv_full[0], 0, p.status, 14, abortw);
-      tc_fence_after();
-      issue_qk(0, 0);
-      issue_qk(0, 1);
-      for (int j = 0; j < NT; ++j) {
-        const int st = j % PF_STAGES;
+      issue_qk(0);
+      if (NT > 1) issue_qk(1);
+      for (int it = 0; it < NT; ++it) {
+        const int st = it % STAGES;
+        tma::mbar_wait(&v_full[st], (it / STAGES) & 1, p.status, 17, abortw);
+        tma::mbar_wait(&p_full[it & 1], (it >> 1) & 1, p.status, 12, abortw);
+        tc_fence_after();
         const uint32_t vbase = smem_u32(sV + st * KV_BYTES);
-        if (j + 1 < NT) tma::mbar_wait(&kv_full[(j + 1) % PF_STAGES], ((j + 1) / PF_STAGES) & 1, p.status, 14, abortw);
+        const uint32_t pcol = tmem + (uint32_t)(it & 1) * PF_BN;      // P (bf16 pairs) sits in the first 32 columns of S
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          tma::mbar_wait(&p_full[s], j & 1, p.status, 12, abortw);
-          tc_fence_after();
-          const uint32_t pcol = tmem + (s ? TM_SN : 0u);          // P (bf16 pairs) sits in the first 64 S columns
-          const uint32_t dcol = tmem + (s ? TM_ON : TM_OS);
-#pragma unroll
-          for (int kk = 0; kk < KSTEPS_PV; ++kk) {
-            const uint64_t bd = smem_desc(vbase + kk * 2048, KV_HALF, 1024);
-            tc_mma_ts(dcol, pcol + kk * 8, bd, IDESC_PV, (j > 0 || kk > 0) ? 1u : 0u);
-          }
-          tc_commit(&pv_done[s]);
-          if (s == 1) tc_commit(&kv_empty[st]);
-          if (j + 1 < NT) issue_qk(j + 1, s);
+        for (int kk = 0; kk < KSTEPS_PV; ++kk) {
+          const uint64_t bd = smem_desc(vbase + kk * 2048, KV_HALF, 1024);
+          tc_mma_ts(tmem + TM_O, pcol + kk * 8, bd, IDESC_PV, (it > 0 || kk > 0) ? 1u : 0u);
         }
+        tc_commit(&pv_done[it & 1]);
+        tc_commit(&v_empty[st]);
+        if (it + 2 < NT) issue_qk(it + 2);
       }
     }
-  }
-    __syncthreads();                                   // every role meets here once all tensor work is done
-    if (warp == 9) {
-      tc_fence_after();
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-    }
-    return;
-  }
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PF_REGS_SOFTMAX));
-  {
-    // =========================== softmax / correction / epilogue (one stream per warp group) ===========================
-    const int s = warp >> 2;                              // 0 = signal, 1 = noise
-    const int sw = warp & 3;                              // warp index inside its group
-    const int quarter = warp & 3;                         // TMEM lane quarter this warp may touch
-    const int row = quarter * 32 + lane;                  // row of the query tile
+  } else {
+    // =========================== softmax / correction / epilogue ===========================
+    const int s = warp >> 1;                              // 0 = signal rows, 1 = noise rows
+    const int row = (warp & 1) * 32 + lane;               // row of the query tile
     const int grow = r0 + row;                            // row inside the block
-    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    const uint32_t s_col = lane_addr + (s ? TM_SN : 0u);
-    const uint32_t o_col = lane_addr + (s ? TM_ON : TM_OS);
-    if (s == 0) {                                         // visibility bits of the prefix slots
-      for (int w32 = sw; w32 < NP * 4; w32 += 4) {
-        const int c = w32 * 32 + lane;
-        const bool vis = c < p.Lbuf && (!p.mask_unused || p.allowed[(long long)b * p.Lbuf + c] != 0);
-        const unsigned bits = __ballot_sync(0xffffffffu, vis);
-        if (lane == 0) sMask[w32] = bits;
-      }
-    }
-    bar_softmax_all();
+    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t o_col = lane_addr + TM_O;
 
     float mb = -INFINITY;                                 // exponent base (lags the true max by < GAP)
     float l = 0.f;
-    for (int j = 0; j < NT; ++j) {
-      tma::mbar_wait(&s_full[s], j & 1, p.status, 16, abortw);
-      tc_fence_after();
+    for (int it = 0; it < NT; ++it) {
+      const uint32_t s_col = lane_addr + (uint32_t)(it & 1) * PF_BN;
       // Visibility per group of 32 keys.  cls: 2 = all visible, 0 = none, 1 = mixed; the class is the same for
       // every lane of a warp: prefix slots carry one mask per state, and in a block tile the 32 rows of a warp
       // meet the causal diagonal inside one group only.
-      uint32_t vis[4]; int cls[4];
-      if (j < NP) {
+      uint32_t vis[2]; int cls[2];
+      if (it < NV) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          vis[q4] = sMask[4 * j + q4];
-          cls[q4] = vis[q4] == 0xffffffffu ? 2 : (vis[q4] == 0u ? 0 : 1);
+        for (int g = 0; g < 2; ++g) {
+          vis[g] = sMask[2 * it + g];
+          cls[g] = vis[g] == 0xffffffffu ? 2 : (vis[g] == 0u ? 0 : 1);
         }
       } else {
-        const int nvis = grow - (j - NP) * PF_BN + 1;     // key c0+i visible iff c0+i <= grow
-        const int qd = (r0 + quarter * 32 - (j - NP) * PF_BN) >> 5;    // group holding this warp's diagonal
+        const int c0 = (it - NV) * PF_BN;
+        const int nvis = grow - c0 + 1;                   // key c0+i visible iff c0+i <= grow
+        const int gd = (r0 + (warp & 1) * 32 - c0) >> 5;  // group holding this warp's diagonal
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int nq = nvis - 32 * q4;
-          vis[q4] = nq >= 32 ? 0xffffffffu : (nq <= 0 ? 0u : ((1u << nq) - 1u));
-          cls[q4] = q4 < qd ? 2 : (q4 == qd ? 1 : 0);
+        for (int g = 0; g < 2; ++g) {
+          const int nq = nvis - 32 * g;
+          vis[g] = nq >= 32 ? 0xffffffffu : (nq <= 0 ? 0u : ((1u << nq) - 1u));
+          cls[g] = g < gd ? 2 : (g == gd ? 1 : 0);
         }
       }
-      // S is read from TMEM once, all 128 keys of the row into registers (TMEM -> register bandwidth, not
-      // arithmetic, bounds a two-pass softmax here); groups without a visible key are not read at all.
-      uint32_t v[4][32];
+      tma::mbar_wait(&s_full[it & 1], (it >> 1) & 1, p.status, 16, abortw);
+      tc_fence_after();
+      // S is read from TMEM once, all 64 keys of the row into registers; groups without a visible key are not read
+      uint32_t v[2][32];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) if (cls[g] != 0) tc_ld32(s_col + g * 32, v[g]);
+      for (int g = 0; g < 2; ++g) if (cls[g] != 0) tc_ld32(s_col + g * 32, v[g]);
       tc_wait_ld();
       // row maximum over the visible keys
       float mx = -INFINITY;
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < 2; ++g) {
         float m0 = -INFINITY, m1 = -INFINITY;
         if (cls[g] == 2) {
 #pragma unroll
@@ -396,10 +387,12 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         mb = mx;
         l *= alpha;
       }
-      // rescale O when some row of this warp moved its exponent base (not for the first tile: the first
-      // P.V overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V
-      if (__any_sync(0xffffffffu, (alpha != 1.f) && j > 0)) {
-        tma::mbar_wait(&pv_done[s], (j - 1) & 1, p.status, 19, abortw);
+      // Rescale O when some row of this warp moved its exponent base (not for the first tile: the first P.V
+      // overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V.  (A barrier per
+      // buffer: s_full of tile it was committed behind P.V it-2, so the barrier of P.V it-1 is at most one phase
+      // behind and its parity is not ambiguous; the same holds for the last P.V in the epilogue.)
+      if (__any_sync(0xffffffffu, (alpha != 1.f) && it > 0)) {
+        tma::mbar_wait(&pv_done[(it - 1) & 1], ((it - 1) >> 1) & 1, p.status, 19, abortw);
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < DH / 16; ++c) {
@@ -417,7 +410,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       const uint64_t scale2 = pk64(p.scale_log2, p.scale_log2), nref2 = pk64(nref, nref);
       uint64_t sum0 = 0ull, sum1 = 0ull, sum2 = 0ull, sum3 = 0ull;     // four independent chains of packed pairs
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
+      for (int g = 0; g < 2; ++g) {
         uint32_t pk[16];
         if (cls[g] == 0) {
 #pragma unroll
@@ -446,81 +439,100 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&p_full[s]);
+      if (lane == 0) tma::mbar_arrive(&p_full[it & 1]);
     }
 
     // ---- epilogue: signal / l_s - lambda * noise / l_n, head RMSNorm, store ----
-    // Both accumulators of a row sit in the same TMEM lane, so a thread reads both streams directly; the two
-    // warp groups split the head dimension (group s takes columns s*Dh/2 ..) and exchange only the row sums
-    // (1/l of each stream, partial sums of squares) through the shared memory of the query tiles, which are
-    // dead once every Q.K^T has completed.  fp32 end to end with a single rounding of the result.
+    // The two streams of a query row sit 64 TMEM lanes apart, in different warps.  Each thread hands one half of its
+    // normalised columns to its partner (signal rows finish columns 0 .. Dh/2-1, noise rows the rest) through the
+    // shared memory of the query tile, which is dead once every Q.K^T has completed; partial sums of squares go
+    // through the K ring and the rounded rows through the V ring, so that a warp stores whole rows.  16-byte chunks
+    // are XORed with the row so that neither the row-wise writes nor the reads collide in a bank.
+    // fp32 end to end with a single rounding of the result.
     const bool valid = grow < p.blk;
     float lam = 0.f;
     if (valid) lam = bf16_round(p.lam[(long long)b * p.lam_bs + (long long)(p.t0 + grow) * p.lam_rs + h]);
     constexpr int HC = DH / 2;                             // columns per thread
-    float nwv[HC];
-    if (p.norm_full) {
+    tma::mbar_wait(&pv_done[(NT - 1) & 1], ((NT - 1) >> 1) & 1, p.status, 18, abortw);
+    tc_fence_after();
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    constexpr int XM = HC / 4 - 1;                         // chunks of 4 floats per exchanged row, minus one
+    float4* xown = reinterpret_cast<float4*>(sQ) + (size_t)(s * PF_BM + row) * (HC / 4);
+    const float4* xpart = reinterpret_cast<const float4*>(sQ) + (size_t)((1 - s) * PF_BM + row) * (HC / 4);
 #pragma unroll
-      for (int i = 0; i < HC / 2; ++i) {
-        const __nv_bfloat162 wv = reinterpret_cast<const __nv_bfloat162*>(p.norm_w)[(s * HC) / 2 + i];
-        nwv[2 * i] = __low2float(wv); nwv[2 * i + 1] = __high2float(wv);
-      }
+    for (int c = 0; c < HC / 32; ++c) {
+      uint32_t o[32];
+      tc_ld32(o_col + (1 - s) * HC + c * 32, o);
+      tc_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        xown[(c * 8 + i) ^ (row & XM)] = make_float4(__uint_as_float(o[4 * i]) * inv, __uint_as_float(o[4 * i + 1]) * inv,
+                                                    __uint_as_float(o[4 * i + 2]) * inv, __uint_as_float(o[4 * i + 3]) * inv);
     }
-    // Each group waits for ITS stream's last P.V only -- a barrier whose phases it has followed in order; a
-    // parity wait on the other stream's barrier could pass on a phase two tiles back.  The block barrier below
-    // then carries "both streams are complete" across the groups.
-    tma::mbar_wait(&pv_done[s], (NT - 1) & 1, p.status, 18, abortw);
-    tc_fence_after();
-    float* xch = reinterpret_cast<float*>(sQs);            // [2][128] 1/l, then [2][128] partial sums of squares
-    xch[s * PF_BM + row] = l > 0.f ? 1.f / l : 0.f;
-    tc_fence_before();
     bar_softmax_all();
-    tc_fence_after();
-    const float inv_s = xch[row], inv_n = xch[PF_BM + row];
     float dv[HC];                                          // sig - lam * noise of this thread's columns
     float sq = 0.f;
 #pragma unroll
     for (int c = 0; c < HC / 32; ++c) {
-      uint32_t os[32], on[32];
-      tc_ld32(lane_addr + TM_OS + s * HC + c * 32, os);
-      tc_ld32(lane_addr + TM_ON + s * HC + c * 32, on);
+      uint32_t o[32];
+      tc_ld32(o_col + s * HC + c * 32, o);
       tc_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float d = fmaf(-lam, __uint_as_float(on[i]) * inv_n, __uint_as_float(os[i]) * inv_s);
-        sq = fmaf(d, d, sq);
-        dv[c * 32 + i] = d;
-      }
-    }
-    xch[2 * PF_BM + s * PF_BM + row] = sq;
-    bar_softmax_all();
-    if (valid) {
-      const float sq_row = xch[2 * PF_BM + row] + xch[3 * PF_BM + row];
-      bf16* op = p.out + (long long)b * p.out_bs + (long long)(p.t0 + grow) * p.out_rs + (long long)h * DH + s * HC;
-      const float rs = p.norm_full ? rsqrtf(sq_row / (float)DH + p.eps) : 1.f;
-#pragma unroll
-      for (int i = 0; i < HC / 8; ++i) {
-        uint32_t w[4];
+      for (int i = 0; i < 8; ++i) {
+        const float4 x = xpart[(c * 8 + i) ^ (row & XM)];
+        const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          float y0 = dv[8 * i + 2 * e] * rs, y1 = dv[8 * i + 2 * e + 1] * rs;
-          if (p.norm_full) { y0 *= nwv[8 * i + 2 * e]; y1 *= nwv[8 * i + 2 * e + 1]; }
-          w[e] = pack2(y0, y1);
+          const float own = __uint_as_float(o[4 * i + e]) * inv;
+          const float d = s == 0 ? fmaf(-lam, xv[e], own) : fmaf(-lam, own, xv[e]);
+          sq = fmaf(d, d, sq);
+          dv[c * 32 + 4 * i + e] = d;
         }
-        reinterpret_cast<uint4*>(op)[i] = make_uint4(w[0], w[1], w[2], w[3]);
       }
+    }
+    float* xsq = reinterpret_cast<float*>(sK);             // [2][64] partial sums of squares
+    xsq[s * PF_BM + row] = sq;
+    if (p.norm_full) bar_softmax_all();
+    const float rs = p.norm_full ? rsqrtf((xsq[row] + xsq[PF_BM + row]) / (float)DH + p.eps) : 1.f;
+    constexpr int RC = DH / 8;                             // 16-byte chunks per output row
+    uint4* srow = reinterpret_cast<uint4*>(sV) + (size_t)row * RC;
+#pragma unroll
+    for (int i = 0; i < HC / 8; ++i) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float y0 = dv[8 * i + 2 * e] * rs, y1 = dv[8 * i + 2 * e + 1] * rs;
+        if (p.norm_full) {
+          const __nv_bfloat162 wv = reinterpret_cast<const __nv_bfloat162*>(p.norm_w)[(s * HC) / 2 + 4 * i + e];
+          y0 *= __low2float(wv); y1 *= __high2float(wv);
+        }
+        w[e] = pack2(y0, y1);
+      }
+      srow[(s * (HC / 8) + i) ^ (row & (RC - 1))] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    bar_softmax_all();
+    bf16* ob = p.out + (long long)b * p.out_bs + (long long)(p.t0 + r0) * p.out_rs + (long long)h * DH;
+#pragma unroll
+    for (int i = 0; i < PF_BM * RC / 128; ++i) {
+      const int x = i * 128 + tid, rr = x / RC, cc = x % RC;
+      if (r0 + rr < p.blk)
+        *reinterpret_cast<uint4*>(ob + (long long)rr * p.out_rs + cc * 8) = reinterpret_cast<const uint4*>(sV)[rr * RC + (cc ^ (rr & (RC - 1)))];
     }
     tc_fence_before();
   }
 
-  __syncthreads();
+  __syncthreads();                                     // every role meets here once all tensor work is done
+  if (warp == 5) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(PF_TMEM_COLS) : "memory");
+  }
 }
 
 template <int DH>
 size_t prefill_smem(int Lbuf) {
   const int NP = (Lbuf + PF_BN - 1) / PF_BN;
-  return (size_t)2 * (DH / 64) * PF_BM * 128 + 2 * PF_STAGES * (size_t)(DH / 64) * PF_BN * 128 +
-         (7 + 2 * PF_STAGES) * 8 + 8 + (size_t)NP * 4 * 4 + 1024 + 64;
+  return (size_t)(DH / 64) * PF_M * 128 + 2 * pf_stages(DH) * (size_t)(DH / 64) * PF_BN * 128 +
+         (7 + 4 * pf_stages(DH)) * 8 + 8 + (size_t)NP * 10 + 1024 + 16;
 }
 
 template <int DH>
@@ -532,15 +544,6 @@ int launch_prefill(const CUtensorMap* maps, const PrefillParams& p, cudaStream_t
     cudaFuncSetAttribute(prefill_attend_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
   });
   dim3 grid((p.blk + PF_BM - 1) / PF_BM, p.H, p.B);
-  {
-    static int pool = 0;
-    if (pool == 0) {
-      cudaFuncAttributes fa;
-      CODA_REQUIRE(cudaFuncGetAttributes(&fa, prefill_attend_kernel<DH>) == cudaSuccess, CODA_ERR_LAUNCH, "prefill_attend: cudaFuncGetAttributes failed");
-      pool = fa.numRegs * PF_THREADS;
-    }
-    CODA_REQUIRE(pool >= PF_REGS_TOTAL, CODA_ERR_LAUNCH, "prefill_attend: register pool %d below the %d the roles ask for", pool, PF_REGS_TOTAL);
-  }
   prefill_attend_kernel<DH><<<grid, PF_THREADS, smem, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
   CODA_CHECK_LAUNCH("prefill_attend");
   return CODA_OK;
