@@ -30,3 +30,45 @@ def test_prefill_attention_at_tile_edges(Dh, H, Hkv, W, Me, Ms, norm, block, L):
     yb, sb = mod.prefill_chunked(x, sb, block_size=block)
     assert torch.equal(sa.k_buf, sb.k_buf) and torch.equal(sa.allowed, sb.allowed)
     assert rel_err(ya, yb) < 8e-3
+
+
+@pytest.mark.parametrize("Dh", [32, 64, 128])
+@pytest.mark.parametrize("Lq,blk,Lbuf,used", [(1, False, 70, 0.5), (1, False, 200, 0.02), (2, True, 33, 0.0), (3, True, 40, 0.6),
+                                              (8, True, 96, 1.0), (9, True, 31, 0.3), (65, True, 130, 0.1), (130, True, 5, 0.0)])
+def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
+    """The register-tiled fp32 kernel (both row counts per tile, keys split over four warps, tiles without a visible key)
+    against the same attention in 64 bits; 32-bit sums over at most 260 keys."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    H, Hkv, B = 4, 2, 2
+    mod = CoDAGQALandmarkPerf2(embed_dim=H * Dh, num_heads=H, num_kv_heads=Hkv, window=Lbuf, num_landmarks_exact=0,
+                               num_landmarks_summary=0).eval().cuda()
+    st = mod.init_state(batch_size=B, device="cuda", dtype=torch.float32)
+    g = torch.Generator("cuda").manual_seed(Dh + Lq + Lbuf)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    st.k_buf.copy_(rnd(*st.k_buf.shape))
+    st.v_buf.copy_(rnd(*st.v_buf.shape))
+    st.allowed.copy_(torch.rand(B, Lbuf, generator=g, device="cuda") < used)
+    q, qn = 2 * rnd(B, Lq, H * Dh), 2 * rnd(B, Lq, H * Dh)
+    lam = torch.rand(B, Lq, H, generator=g, device="cuda")
+    k, v = (rnd(B, Lq, Hkv * Dh), rnd(B, Lq, Hkv * Dh)) if blk else (None, None)
+    with torch.no_grad():
+        mod.head_norm.weight.copy_(rnd(Dh))
+    out = torch.full((B, Lq, H * Dh), float("nan"), device="cuda")
+    mod._attend(mod._cfg(B, torch.float32, st), st, Lq, q, qn, lam, k, v, out)
+
+    d = lambda t: t.double()  # noqa: E731
+    keys, vals = d(st.k_buf), d(st.v_buf)
+    vis = st.allowed.bool()[:, None, :].expand(B, Lq, Lbuf)
+    if blk:
+        keys = torch.cat([keys, d(k).view(B, Lq, Hkv, Dh).transpose(1, 2)], 2)
+        vals = torch.cat([vals, d(v).view(B, Lq, Hkv, Dh).transpose(1, 2)], 2)
+        vis = torch.cat([vis, torch.ones(Lq, Lq, device="cuda").tril().bool().expand(B, Lq, Lq)], 2)
+    keys, vals = (t.repeat_interleave(H // Hkv, 1) for t in (keys, vals))
+
+    def stream(x):
+        s = d(x).view(B, Lq, H, Dh).transpose(1, 2) @ keys.transpose(2, 3) / Dh ** 0.5
+        return torch.softmax(s.masked_fill(~vis[:, None], float("-inf")), -1).nan_to_num(0.0) @ vals
+
+    y = stream(q) - d(lam).transpose(1, 2)[..., None] * stream(qn)
+    y = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + mod.eps) * d(mod.head_norm.weight)
+    assert rel_err(out, y.transpose(1, 2).reshape(B, Lq, H * Dh)) < 5e-6
