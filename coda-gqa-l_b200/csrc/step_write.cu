@@ -305,11 +305,15 @@ __global__ void __launch_bounds__(512) step_write_kernel(StepParams p) {
 // bulk copies issued by the first thread at entry instead of into registers by every thread: the scoring loop
 // reads them from there, no thread holds cache chunks across the entry phase, and more CTAs fit an SM.  The
 // launcher adds their bytes (rounded up to 16) to the dynamic shared memory and picks STAGE only when they fit.
-template <typename T, int DH, int MODE, bool STAGE = false>
+//
+// NT: threads per CTA, at least one per element of the head's K and V rows.
+template <typename T, int DH, int MODE, bool STAGE = false, int NT = 256>
 __device__ __forceinline__ void step_cluster_body(const StepParams& p) {
   constexpr bool ROUTE = MODE != 2, APPEND = MODE != 1;
   static_assert(!STAGE || MODE == 1, "staged caches are for the routing-only launch");
-  constexpr int NT = 256, LF = DH / 2, LFD = DH - LF;
+  static_assert(NT >= 2 * DH && NT >= 64, "a thread per element of the K and V rows, a warp per bank");
+  constexpr int LF = DH / 2, LFD = DH - LF;
+  constexpr int PA = 1024 / NT, PL = 256 / NT;            // slot flags and LRU stamps per thread (Lbuf <= 1024, Me <= 256)
   constexpr int EPV = 16 / (int)sizeof(T);                // elements per 16-byte chunk
   constexpr int CE = DH / EPV, CS = LFD / EPV;            // chunks per exact / summary routing-cache row (powers of two <= 32)
   constexpr int PE = 4, PS = 2;                           // chunks per thread requested at kernel entry
@@ -379,11 +383,13 @@ __device__ __forceinline__ void step_cluster_body(const StepParams& p) {
     for (int j = 0; j < PS; ++j) ps[j] = (ROUTE && tid + j * NT < ncs) ? kn4[tid + j * NT] : make_uint4(0u, 0u, 0u, 0u);
   }
   // slot flags and LRU stamps: requested into registers now, parked in shared memory once every other request
-  // is out (a load -> shared-store loop would cost one memory round trip per loop); Lbuf <= 4 * NT, Me <= NT
-  uint8_t alr[4];
+  // is out (a load -> shared-store loop would cost one memory round trip per loop)
+  uint8_t alr[PA];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) { const int m = tid + a * NT; alr[a] = m < Lbuf ? al[m] : (uint8_t)0; }
-  const long long lastr = (ROUTE && tid < Me) ? ((const long long*)p.st.mem_last_exact)[(long long)b * Me + tid] : 0;
+  for (int a = 0; a < PA; ++a) { const int m = tid + a * NT; alr[a] = m < Lbuf ? al[m] : (uint8_t)0; }
+  long long lastr[PL];
+#pragma unroll
+  for (int a = 0; a < PL; ++a) { const int m = tid + a * NT; lastr[a] = (ROUTE && m < Me) ? ((const long long*)p.st.mem_last_exact)[(long long)b * Me + m] : 0; }
   // the new token's row (element tid < DH: key, DH <= tid < 2*DH: value)
   T nk_a_raw = T(), nk_b_raw = T(), glog_raw = T();
   float nv_x = 0.f, eta_raw = 0.f, glog = 0.f;
@@ -493,8 +499,9 @@ __device__ __forceinline__ void step_cluster_body(const StepParams& p) {
     if (is_v) ve[d] = El<T>::ld(&ve_raw);
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a) { const int m = tid + a * NT; if (m < Lbuf) s_al[m] = alr[a]; }
-  if (tid < Me) s_last[tid] = lastr;
+  for (int a = 0; a < PA; ++a) { const int m = tid + a * NT; if (m < Lbuf) s_al[m] = alr[a]; }
+#pragma unroll
+  for (int a = 0; a < PL; ++a) { const int m = tid + a * NT; if (m < Me) s_last[m] = lastr[a]; }
   __syncthreads();
   // rotated key element d (primitives.py:99-113)
   float new_k = nk_a;
@@ -957,14 +964,16 @@ __global__ void __launch_bounds__(256) step_write_cluster_kernel(StepParams p) {
 // Routing (MODE 1) of MANY layers' states in one launch: blockIdx.z picks the layer's parameter block from a
 // device array.  The routing of one layer is a latency chain that keeps an SM's resources while it waits; all
 // layers' chains side by side fill the machine and are bounded by memory bandwidth instead.
-template <typename T, int DH, bool STAGE, int NCTA>
-__global__ void __launch_bounds__(256, NCTA) step_route_batched_kernel(const StepParams* __restrict__ layers) {
+// The chain is as long with 128 threads as with 256 and a CTA needs no more of them at Dh 64, so there twice as many
+// chains share an SM: 122 -> 86 us for 8 layers x 512 states x 3 heads.
+template <typename T, int DH, bool STAGE, int NCTA, int NT>
+__global__ void __launch_bounds__(NT, NCTA) step_route_batched_kernel(const StepParams* __restrict__ layers) {
   __shared__ StepParams sp;
   static_assert(sizeof(StepParams) % 4 == 0, "StepParams is copied word by word");
   const uint32_t* src = reinterpret_cast<const uint32_t*>(layers + blockIdx.z);
-  for (int i = threadIdx.x; i < (int)(sizeof(StepParams) / 4); i += 256) reinterpret_cast<uint32_t*>(&sp)[i] = src[i];
+  for (int i = threadIdx.x; i < (int)(sizeof(StepParams) / 4); i += NT) reinterpret_cast<uint32_t*>(&sp)[i] = src[i];
   __syncthreads();
-  step_cluster_body<T, DH, 1, STAGE>(sp);
+  step_cluster_body<T, DH, 1, STAGE, NT>(sp);
 }
 
 template <typename T, int DH, int MODE>
@@ -1175,7 +1184,7 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
   const int MM = cfg->Me + cfg->Ms;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(cfg->Hkv, cfg->B, n_layers);
-  lc.blockDim = dim3(256, 1, 1);
+  lc.blockDim = dim3(cfg->Dh == 128 ? 256 : 128, 1, 1);
   lc.dynamicSmemBytes = sizeof(float) * ((size_t)cfg->Hkv * MM + MM) + 8 + 8 * (size_t)cfg->Me + (size_t)(cfg->W + MM) + 16;
   lc.stream = (cudaStream_t)stream;
   cudaLaunchAttribute at[1];
@@ -1191,11 +1200,11 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
   if (stage) {
     lc.dynamicSmemBytes += 16 + stage_bytes;
     // five CTAs per SM measured best at the 7B shape (4: 122 us, 5: 111 us, 6: 114 us for 32 layers x 32 states)
-    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, true, 5>, plan)
-                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 5>, plan);
+    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, true, 5, 256>, plan)
+                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 10, 128>, plan);
   } else {
-    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, false, 4>, plan)
-                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 4>, plan);
+    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, false, 4, 256>, plan)
+                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 8, 128>, plan);
   }
   if (e != cudaSuccess) { coda_set_error("step_route_batched: %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
   return CODA_OK;

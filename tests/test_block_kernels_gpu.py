@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from tests.helpers import orc, rel_err
+from tests.helpers import TOL_BF16, orc, rel_err
 from tests.scenarios import randomize_weights
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +72,44 @@ def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
     y = stream(q) - d(lam).transpose(1, 2)[..., None] * stream(qn)
     y = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + mod.eps) * d(mod.head_norm.weight)
     assert rel_err(out, y.transpose(1, 2).reshape(B, Lq, H * Dh)) < 5e-6
+
+
+@pytest.mark.parametrize("kw,B", [
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=700, num_landmarks_exact=140, num_landmarks_summary=60), 2),
+    (dict(embed_dim=192, num_heads=3, num_kv_heads=3, window=32, num_landmarks_exact=32, num_landmarks_summary=32), 150),
+    (dict(embed_dim=512, num_heads=8, num_kv_heads=1, window=33, num_landmarks_exact=5, num_landmarks_summary=90), 7),
+])
+def test_batched_routing_head_dim_64(kw, B):
+    """128-thread CTAs of the all-layers routing launch (more slots, stamps and cache chunks than threads), through the captured step against eager steps: the same bits in both banks."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, CoDAStack, _deep_copy_state
+    torch.manual_seed(5)
+    layers = [CoDAGQALandmarkPerf2(**kw).eval() for _ in range(2)]
+    for i, layer in enumerate(layers):
+        randomize_weights(layer, 5 + i)
+    layers = [layer.to(torch.bfloat16).cuda() for layer in layers]
+    T, D = kw["window"] + 150, kw["embed_dim"]
+    x = orc.mixture_inputs(B, T + 20, D, centroids=16, sigma=0.3, seed=8, dtype=torch.bfloat16).cuda()
+    states = []
+    for layer in layers:
+        st = layer.init_state(batch_size=B, device="cuda", dtype=torch.bfloat16)
+        layer.prefill_chunked(x[:, :T], st, block_size=64, return_outputs=False)
+        states.append(st)
+    twins = [_deep_copy_state(s) for s in states]
+    stack = CoDAStack(layers)
+    tok = x[:, T:T + 1].contiguous()
+    stack.capture_step(states, tok)
+    for t in range(T, T + 20):
+        tok = x[:, t:t + 1].contiguous()
+        y = stack.step_graph(tok, states)
+        h = tok
+        for layer, st in zip(layers, twins):
+            o, _ = layer.step(h, st)
+            h = h + o
+        assert rel_err(y, h) < TOL_BF16
+    # (the captured projections may round elsewhere, but every token evicted here was written by the shared prefill)
+    W = kw["window"]
+    for a, b in zip(states, twins):
+        assert torch.equal(a.allowed, b.allowed) and torch.equal(a.mem_last_exact, b.mem_last_exact)
+        assert torch.equal(a.k_buf[:, :, W:], b.k_buf[:, :, W:]) and torch.equal(a.v_buf[:, :, W:], b.v_buf[:, :, W:])
+        assert torch.equal(a._exact_v_norm, b._exact_v_norm) and torch.equal(a._sum_lf_k_norm, b._sum_lf_k_norm)
+    assert all(layer.device_status() == 0 for layer in layers)
