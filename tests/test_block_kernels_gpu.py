@@ -80,7 +80,8 @@ def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
     (dict(embed_dim=512, num_heads=8, num_kv_heads=1, window=33, num_landmarks_exact=5, num_landmarks_summary=90), 7),
 ])
 def test_batched_routing_head_dim_64(kw, B):
-    """128-thread CTAs of the all-layers routing launch (more slots, stamps and cache chunks than threads), through the captured step against eager steps: the same bits in both banks."""
+    """128-thread CTAs of the all-layers routing launch (more slots, stamps and cache chunks than threads) and two attention
+    CTAs per SM, through the captured step against eager steps: the same bits in both banks."""
     from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, CoDAStack, _deep_copy_state
     torch.manual_seed(5)
     layers = [CoDAGQALandmarkPerf2(**kw).eval() for _ in range(2)]
