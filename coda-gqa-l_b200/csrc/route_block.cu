@@ -8,7 +8,7 @@
 //   ring_rewrite  grid (2*Hkv, B): kept ring rows shift to the front, the block's tail is appended.
 // Semantics: upstream memory_banks.py:438-564 (block write), 633-742 (exact), 853-932 (summary).
 #include "coda_common.cuh"
-#include "topk_order.h"
+#include "topk_warp.cuh"
 #include "tma_utils.cuh"
 #include "bank_score.cuh"
 #include <mutex>
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(256) route_score_heads_kernel(RouteParams p) {
 // Per-state plan written by route_decide and consumed by route_apply (all int32 / fp32, in global scratch).
 struct Plan {
   int* e_tgt; int* e_flag;            // [Te]  target slot; bit0 overwrite, bit1 touch, bit2 first overwriter of its slot
-  float* s_w; int* s_ord;             // [Ts]  summary weights; candidates grouped by slot
+  float* s_w; int* s_ord;             // [Ts]  summary weights and evicted indices, grouped by slot in candidate order
   int* s_start; float* s_cnt; int* s_was;   // [Ms+1], [Ms], [Ms]
 };
 __device__ __forceinline__ Plan plan_of(const RouteParams& p, int b) {
@@ -376,35 +376,40 @@ __device__ __forceinline__ Plan plan_of(const RouteParams& p, int b) {
 }
 
 // ---- decisions: the order-dependent part, one small CTA per state ----
-// Inputs are staged into shared memory by all threads, the two serial sections (exact bank on thread 0,
-// summary bank on thread 32) work on shared memory only, and the plan is copied out cooperatively.
+// Warp 0 decides for the exact bank, the other warps keep the summary bank's books.  What looks serial is a prefix
+// count or a per-slot extremum: the rank of a novel candidate is the number of novel kept candidates up to it, the
+// first overwriter of a slot is the smallest candidate index and its stamp the largest position among those that
+// touch it (shared-memory min / max: independent of the order).  Only a slot's weight sum is rounded after each term; a
+// thread per slot walks the candidates for it.
+// Bound: latency of one short CTA per state; one thread walking these loops in shared memory took
+// 23 us per block for 64 states (256-token blocks, 8 + 64 candidates), this 9 us.
+constexpr int RD_THREADS = 160;
+
 template <typename T>
-__global__ void __launch_bounds__(64) route_decide_kernel(RouteParams p) {
-  extern __shared__ unsigned char smraw[];
+__global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   const coda_layer_cfg& c = p.c;
-  const int b = blockIdx.x, tid = threadIdx.x, NT = blockDim.x;
+  const int b = blockIdx.x, tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
   const int Me = c.Me, Ms = c.Ms, W = c.W, Lbuf = W + Me + Ms;
   const int te = (Me > 0) ? p.te : 0, ts = (Ms > 0) ? p.ts : 0, tmax = te > ts ? te : ts;
   typedef topk_order::Item<long long> It64;
   It64* lruq = reinterpret_cast<It64*>(smraw);                       // [Me]
   long long* s_last = reinterpret_cast<long long*>(lruq + (Me > 0 ? Me : 1));   // [Me]
-  long long* n_last = s_last + (Me > 0 ? Me : 1);                    // [Me] new stamps
-  float* c_g = reinterpret_cast<float*>(n_last + (Me > 0 ? Me : 1)); // [tmax] gates
+  float* c_g = reinterpret_cast<float*>(s_last + (Me > 0 ? Me : 1)); // [tmax] gates
   float* x_best = c_g + (tmax > 0 ? tmax : 1);                       // [te]
   float* w_s = x_best + (te > 0 ? te : 1);                           // [ts] summary weights
-  float* cnt_s = w_s + (ts > 0 ? ts : 1);                            // [Ms]
-  int* c_e = reinterpret_cast<int*>(cnt_s + (Ms > 0 ? Ms : 1));      // [tmax] evicted index
+  int* c_e = reinterpret_cast<int*>(w_s + (ts > 0 ? ts : 1));        // [tmax] evicted index
   int* x_bi = c_e + (tmax > 0 ? tmax : 1);                           // [te]
-  int* tgt_s = x_bi + (te > 0 ? te : 1);                             // [te]
-  int* flag_s = tgt_s + (te > 0 ? te : 1);                           // [te]
-  int* s_idx = flag_s + (te > 0 ? te : 1);                           // [ts]
-  int* ord_s = s_idx + (ts > 0 ? ts : 1);                            // [ts]
-  int* start_s = ord_s + (ts > 0 ? ts : 1);                          // [Ms+1]
-  int* s_cur = start_s + Ms + 1;                                     // [Ms]
-  unsigned char* s_used = reinterpret_cast<unsigned char*>(s_cur + (Ms > 0 ? Ms : 1));   // [Me + Ms]
+  int* s_idx = x_bi + (te > 0 ? te : 1);                             // [ts]
+  int* n_first = s_idx + (ts > 0 ? ts : 1);                          // [Me] first overwriting candidate of a slot
+  int* n_e = n_first + (Me > 0 ? Me : 1);                            // [Me] largest touching evicted index, -1: none
+  int* start_s = n_e + (Me > 0 ? Me : 1);                            // [Ms+1]
+  uint16_t* qscr = reinterpret_cast<uint16_t*>(start_s + Ms + 1);    // [2*Me] partition scratch
+  unsigned char* s_used = reinterpret_cast<unsigned char*>(qscr + 2 * (Me > 0 ? Me : 1));   // [Me + Ms]
   const uint8_t* al = p.st.allowed + (long long)b * Lbuf;
   long long* last = (long long*)p.st.mem_last_exact + (long long)b * Me;
   Plan pl = plan_of(p, b);
+  const int Ae = c.active_exact;
   for (int t = tid; t < tmax; t += NT) {
     const int e = p.cand[(long long)b * p.cand_bs + t];
     c_e[t] = e;
@@ -412,223 +417,298 @@ __global__ void __launch_bounds__(64) route_decide_kernel(RouteParams p) {
   }
   for (int t = tid; t < te; t += NT) { x_best[t] = p.ex_best[(long long)b * c.Te + t]; x_bi[t] = p.ex_bi[(long long)b * c.Te + t]; }
   for (int t = tid; t < ts; t += NT) s_idx[t] = p.su_idx[(long long)b * c.Ts + t];
-  for (int m = tid; m < Me + Ms; m += NT) s_used[m] = al[W + m];
-  for (int m = tid; m < Me; m += NT) { s_last[m] = last[m]; n_last[m] = last[m]; }
-  __syncthreads();
-
-  // routing-event record of this call (optional): cleared here, filled by the two deciding threads below
+  for (int m = tid; m < Ms; m += NT) s_used[Me + m] = al[W + Me + m];
+  int used_here = 0;
+  for (int m = tid; m < Me; m += NT) {
+    const bool used = al[W + m] != 0;
+    const long long stamp = last[m];
+    s_used[m] = used;
+    s_last[m] = stamp;
+    lruq[m].v = (used && m < Ae) ? stamp : -(1LL << 62);
+    lruq[m].i = m;
+    n_first[m] = 0x7fffffff; n_e[m] = -1;
+    used_here |= used ? 1 : 0;
+  }
+  // routing-event record of this call (optional): cleared here, filled by the deciding warps below
   int32_t* evw = p.st.events != nullptr ? p.st.events + (long long)b * CODA_EVENT_WORDS : nullptr;
   if (evw != nullptr && tid < CODA_EVENT_WORDS) evw[tid] = 0;
-  __syncthreads();
-  if (tid == 0 && te > 0) {
-    // ---- exact bank (memory_banks.py:635-697) ----
-    const int Ae = c.active_exact;
-    int n_gated = 0, n_hit = 0, n_ins = 0, n_ow = 0, n_frus = 0;
-    bool any_used = false;
-    for (int m = 0; m < Me; ++m) {
-      const bool used = s_used[m] != 0;
-      any_used |= used;
-      lruq[m].v = (used && m < Ae) ? s_last[m] : -(1LL << 62);
-      lruq[m].i = m;
-    }
-    const int n_lru = te < Ae ? te : Ae;
-    topk_order::topk_queue<long long, false>(lruq, Me, n_lru, true);   // victims = lruq[0..n_lru).i
-    const float tn = El<T>::rnd(c.tau_novel), tm = El<T>::rnd(c.tau_match);
-    int rank = -1;
-    for (int t = 0; t < te; ++t) {
-      const float best = x_best[t];
-      const bool keep = c.gated ? (c_g[t] >= c.tau_gate_exact) : true;
-      const bool novel = !any_used || best < tn;
-      const bool hit = any_used && best >= tm;
-      const bool nk = novel && keep;
-      if (nk) ++rank;
-      const bool capped = nk && rank < Ae;
-      int r = rank < 0 ? 0 : rank;
-      if (r > n_lru - 1) r = n_lru - 1 > 0 ? n_lru - 1 : 0;
-      const int tgt = capped ? lruq[r].i : x_bi[t];
-      const bool touch = keep && (!novel || capped);
-      const bool ow = c.refresh_on_hit ? (keep && (capped || hit)) : capped;
-      int flag = (ow ? 1 : 0) | (touch ? 2 : 0);
-      if (ow) {
-        bool first = true;
-        for (int u = 0; u < t; ++u) if ((flag_s[u] & 1) && tgt_s[u] == tgt) { first = false; break; }
-        if (first) flag |= 4;
+  const bool any_used = __syncthreads_or(used_here) != 0;
+  if (tid < 32) {
+    if (te > 0) {
+      // ---- exact bank (memory_banks.py:635-697) ----
+      const int n_lru = te < Ae ? te : Ae;
+      topk_order::topk_queue_warp<long long, false>(lruq, Me, n_lru, true, qscr);   // victims = lruq[0..n_lru).i
+      const float tn = El<T>::rnd(c.tau_novel), tm = El<T>::rnd(c.tau_match);
+      int ranked = 0, n_gated = 0, n_hit = 0, n_ins = 0, n_ow = 0, n_frus = 0;
+      for (int t0 = 0; t0 < te; t0 += 32) {
+        const int t = t0 + lane;
+        const bool in = t < te;
+        const float best = in ? x_best[t] : 0.f;
+        const bool keep = in && (c.gated ? (c_g[t] >= c.tau_gate_exact) : true);
+        const bool novel = !any_used || best < tn;
+        const bool hit = any_used && best >= tm;
+        const bool nk = novel && keep;
+        const unsigned nkb = __ballot_sync(0xffffffffu, nk);
+        const int rank = ranked + __popc(nkb & (0xffffffffu >> (31 - lane))) - 1;
+        ranked += __popc(nkb);
+        const bool capped = nk && rank < Ae;
+        int r = rank < 0 ? 0 : rank;
+        if (r > n_lru - 1) r = n_lru - 1 > 0 ? n_lru - 1 : 0;
+        const int tgt = capped ? lruq[r].i : (in ? x_bi[t] : 0);
+        const bool touch = keep && (!novel || capped);
+        const bool ow = c.refresh_on_hit ? (keep && (capped || hit)) : capped;
+        if (ow) atomicMin(&n_first[tgt], t);
+        if (touch) atomicMax(&n_e[tgt], c_e[t]);
+        __syncwarp();
+        // (an earlier chunk's candidates are in already, a later one's are larger: the minimum is final for this chunk)
+        if (in) { pl.e_tgt[t] = tgt; pl.e_flag[t] = (ow ? 1 : 0) | (touch ? 2 : 0) | (ow && n_first[tgt] == t ? 4 : 0); }
+        if (evw != nullptr) {
+          n_gated += __popc(__ballot_sync(0xffffffffu, in && c.gated && !keep)); n_hit += __popc(__ballot_sync(0xffffffffu, hit && keep));
+          n_ins += __popc(__ballot_sync(0xffffffffu, capped)); n_ow += __popc(__ballot_sync(0xffffffffu, ow));
+          n_frus += __popc(__ballot_sync(0xffffffffu, nk && !capped));
+        }
       }
-      tgt_s[t] = tgt;
-      flag_s[t] = flag;
-      n_gated += (c.gated && !keep) ? 1 : 0; n_hit += (hit && keep) ? 1 : 0; n_ins += capped ? 1 : 0;
-      n_ow += ow ? 1 : 0; n_frus += (nk && !capped) ? 1 : 0;
-    }
-    if (evw != nullptr) { evw[0] = n_gated; evw[1] = n_hit; evw[2] = n_ins; evw[3] = n_ow; evw[4] = n_frus; }
-    // stamps: per slot the largest position among touching candidates replaces the old stamp (:682-697)
-    for (int t = 0; t < te; ++t) {
-      if (!(flag_s[t] & 2)) continue;
-      const int tgt = tgt_s[t];
-      bool first = true;
-      for (int u = 0; u < t; ++u) if ((flag_s[u] & 2) && tgt_s[u] == tgt) { first = false; break; }
-      if (!first) continue;
-      long long mx = p.pos_first + c_e[t];
-      for (int u = t + 1; u < te; ++u)
-        if ((flag_s[u] & 2) && tgt_s[u] == tgt) { const long long pu = p.pos_first + c_e[u]; if (pu > mx) mx = pu; }
-      n_last[tgt] = mx;
-    }
-  }
-  if (tid == 32 && ts > 0) {
-    // ---- summary bank bookkeeping (memory_banks.py:880-885, 906): weights, per-slot candidate lists ----
-    for (int m = 0; m < Ms; ++m) { cnt_s[m] = 0.f; start_s[m] = 0; }
-    start_s[Ms] = 0;
-    for (int t = 0; t < ts; ++t) {
-      float w = El<T>::rnd(c_g[t]);
-      if (c.gated && !(c_g[t] >= c.tau_gate_summary)) w = 0.f;           // (:518-523)
-      w_s[t] = w;
-      const int m = s_idx[t];
-      cnt_s[m] = t_add<T>(cnt_s[m], w);
-      start_s[m + 1] += 1;
-    }
-    for (int m = 0; m < Ms; ++m) start_s[m + 1] += start_s[m];
-    for (int m = 0; m < Ms; ++m) s_cur[m] = start_s[m];
-    for (int t = 0; t < ts; ++t) ord_s[s_cur[s_idx[t]]++] = t;            // stable grouping by slot
-    if (evw != nullptr) {
-      const int As = c.active_summary;
-      int n_upd = 0, n_new = 0; bool all_used = true, incoming = false;
-      for (int m = 0; m < Ms; ++m) {
-        const bool got = cnt_s[m] > 0.f, was = s_used[Me + m] != 0;
-        n_upd += got ? 1 : 0; n_new += (got && !was) ? 1 : 0;
-        if (m < As) { all_used = all_used && (was || got); incoming = incoming || got; }
+      if (evw != nullptr && lane == 0) { evw[0] = n_gated; evw[1] = n_hit; evw[2] = n_ins; evw[3] = n_ow; evw[4] = n_frus; }
+      __syncwarp();
+      // stamps: per slot the largest position among touching candidates replaces the old stamp (:682-697)
+      for (int m = lane; m < Me; m += 32) {
+        if (n_e[m] < 0) continue;
+        const long long stamp = p.pos_first + n_e[m];
+        if (stamp != s_last[m]) last[m] = stamp;
       }
-      evw[5] = n_upd; evw[6] = n_new; evw[7] = all_used ? 1 : 0; evw[8] = incoming ? 1 : 0;
     }
+    return;
   }
-  __syncthreads();
-  for (int t = tid; t < te; t += NT) { pl.e_tgt[t] = tgt_s[t]; pl.e_flag[t] = flag_s[t]; }
-  for (int m = tid; m < Me; m += NT) if (te > 0 && n_last[m] != s_last[m]) last[m] = n_last[m];
-  for (int t = tid; t < ts; t += NT) { pl.s_w[t] = w_s[t]; pl.s_ord[t] = ord_s[t]; }
-  if (ts > 0) {
-    for (int m = tid; m <= Ms; m += NT) pl.s_start[m] = start_s[m];
-    for (int m = tid; m < Ms; m += NT) { pl.s_cnt[m] = cnt_s[m]; pl.s_was[m] = s_used[Me + m] != 0; }
+  if (ts <= 0) return;
+  // ---- summary bank bookkeeping (memory_banks.py:880-885, 906): weights, per-slot candidate lists ----
+  constexpr int NS = RD_THREADS - 32;
+  const int sid = tid - 32;
+  auto sync_s = [] { asm volatile("bar.sync 1, %0;" ::"n"(NS) : "memory"); };
+  for (int t = sid; t < ts; t += NS) {
+    float w = El<T>::rnd(c_g[t]);
+    if (c.gated && !(c_g[t] >= c.tau_gate_summary)) w = 0.f;             // (:518-523)
+    w_s[t] = w;
+  }
+  sync_s();
+  for (int m = sid; m < Ms; m += NS) {
+    float cnt = 0.f;
+    int n = 0;
+#pragma unroll 4
+    for (int t = 0; t < ts; ++t)
+      if (s_idx[t] == m) { cnt = t_add<T>(cnt, w_s[t]); ++n; }
+    pl.s_cnt[m] = cnt;
+    pl.s_was[m] = s_used[Me + m] != 0;
+    start_s[m + 1] = n;
+    s_used[Me + m] = (s_used[Me + m] != 0 ? 1 : 0) | (cnt > 0.f ? 2 : 0);    // for the event record
+  }
+  if (sid == 0) start_s[0] = 0;
+  sync_s();
+  if (tid < 64) {                                                        // inclusive prefix sum over the slots
+    int carry = 0;
+    for (int m0 = 1; m0 <= Ms; m0 += 32) {
+      int v = m0 + lane <= Ms ? start_s[m0 + lane] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+      v += carry;
+      if (m0 + lane <= Ms) start_s[m0 + lane] = v;
+      carry = __shfl_sync(0xffffffffu, v, 31);
+    }
+  } else if (tid < 96 && evw != nullptr) {
+    const int As = c.active_summary;
+    int n_upd = 0, n_new = 0; bool all_used = true, incoming = false;
+    for (int m = lane; m < Ms; m += 32) {
+      const bool got = (s_used[Me + m] & 2) != 0, was = (s_used[Me + m] & 1) != 0;
+      n_upd += got ? 1 : 0; n_new += (got && !was) ? 1 : 0;
+      if (m < As) { all_used = all_used && (was || got); incoming = incoming || got; }
+    }
+    n_upd = __reduce_add_sync(0xffffffffu, n_upd); n_new = __reduce_add_sync(0xffffffffu, n_new);
+    all_used = __all_sync(0xffffffffu, all_used); incoming = __any_sync(0xffffffffu, incoming);
+    if (lane == 0) { evw[5] = n_upd; evw[6] = n_new; evw[7] = all_used ? 1 : 0; evw[8] = incoming ? 1 : 0; }
+  }
+  sync_s();
+  for (int m = sid; m <= Ms; m += NS) pl.s_start[m] = start_s[m];
+  for (int m = sid; m < Ms; m += NS) {                                   // stable grouping by slot
+    int a = start_s[m];
+    if (start_s[m + 1] == a) continue;
+#pragma unroll 4
+    for (int t = 0; t < ts; ++t)
+      if (s_idx[t] == m) { pl.s_ord[a] = c_e[t]; pl.s_w[a] = w_s[t]; ++a; }
   }
 }
 
-// ---- slot writes: one CTA per written slot (exact: per overwriting candidate group; summary: per slot) ----
-// Each thread owns runs of 8 consecutive elements of the slot's [Hkv*Dh] row pair and loads old values and
-// candidate rows in batches.
-template <typename T>
-__global__ void __launch_bounds__(128) route_apply_kernel(RouteParams p) {
-  extern __shared__ float stash[];                                   // [Hkv*Dh] new row for re-normalising, then the slot's candidate list
+// ---- slot writes ----
+// One group of WPS warps per written slot (exact: per overwriting candidate group; summary: per slot).  The slot's K
+// and V rows are cut into 8-element chunks, each owned by one thread, which reads the old values and the candidates'
+// rows (NB candidates in flight) and adds them in list order.  The candidate list is read 32 at a time by the lanes of
+// every warp and handed round by shuffles.
+// In bf16 the sums are packed: one instruction per element pair for the weighted row and one for the sum, each result the
+// rounding of the exact value, which is what the reference's op-by-op bf16 arithmetic gives.
+// A group has a thread for each chunk of rows of up to 1024 elements over all heads (one warp up to 128 elements, two up
+// to 256, else eight; larger rows loop), so that old rows and candidates are one round trip.  A CTA per slot of a narrow
+// layer left three threads in four idle and the chip waiting on CTA launches.
+// Per block: 40 -> 12.5 us (64 states, 2 x 64 elements a row), 233 -> 91 us (512 states, 3 x 64), 31 -> 22 us (32 states, 8 x 128).
+template <typename T, int WPS, bool PACKED>
+__global__ void __launch_bounds__(WPS == 8 ? 256 : 128, WPS == 8 ? 3 : 6) route_apply_kernel(RouteParams p, int nslots) {
+  extern __shared__ float stash_all[];                               // [groups of the CTA][Hkv*Dh] new rows for re-normalising
   const coda_layer_cfg& c = p.c;
-  const int b = blockIdx.y, tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5, NW = NT >> 5;
+  constexpr int GT = 32 * WPS, GROUPS = (WPS == 8 ? 256 : 128) / GT; // threads of a slot's group, groups per CTA
+  const int b = blockIdx.y, lane = threadIdx.x & 31, gid = threadIdx.x / GT, tid = threadIdx.x % GT;
+  const int job = blockIdx.x * GROUPS + gid;
+  if (job >= nslots) return;
   const int Hkv = c.Hkv, Dh = c.Dh, HD = Hkv * Dh, lf = Dh / 2, lfd = Dh - lf;
-  // Every candidate of the block may land on one slot (a one-slot summary bank, clustered keys), so the list
-  // staged per slot holds max(te, ts) entries: nothing is ever dropped from a slot's sum.
-  const int TMAX = max(max(p.te, p.ts), 1);
-  int* s_cand = reinterpret_cast<int*>(stash + HD);
-  float* s_wt = reinterpret_cast<float*>(s_cand + TMAX);
+  float* stash = stash_all + gid * HD;
   const int Me = c.Me, Ms = c.Ms, W = c.W, Lbuf = W + Me + Ms;
   const int te = (Me > 0) ? p.te : 0;
-  uint8_t* al = p.st.allowed + (long long)b * Lbuf;
-  T* kb = (T*)p.st.k_buf + (long long)b * Hkv * Lbuf * Dh;
-  T* vb = (T*)p.st.v_buf + (long long)b * Hkv * Lbuf * Dh;
   const Plan pl = plan_of(p, b);
-  __shared__ int s_n;
-  const bool exact = (int)blockIdx.x < te;
-  int slot;                                                          // slot index inside its bank
+  const bool exact = job < te;
+  int slot, first, last;                                             // slot of its bank; range of the list scanned for it
   float cden = 1.f; bool fresh = false;
   if (exact) {
     // ---- exact bank write (memory_banks.py:707-742): candidates that overwrite this slot, in list order ----
-    const int t = blockIdx.x;
-    if ((pl.e_flag[t] & 5) != 5) return;                               // not the first overwriter of its slot
-    slot = pl.e_tgt[t];
-    if (tid == 0) {
-      int nn = 0;
-      for (int u = t; u < te; ++u)
-        if ((pl.e_flag[u] & 1) && pl.e_tgt[u] == slot) { s_cand[nn] = p.cand[(long long)b * p.cand_bs + u]; s_wt[nn] = 1.f; ++nn; }
-      s_n = nn;
-    }
+    if ((pl.e_flag[job] & 5) != 5) return;                           // not the first overwriter of its slot
+    slot = pl.e_tgt[job];
+    first = job; last = te;
   } else {
     // ---- summary bank EMA of one slot (memory_banks.py:887-932) ----
-    slot = blockIdx.x - te;
-    if (slot >= Ms || p.ts <= 0) return;
+    slot = job - te;
     const float cnt = pl.s_cnt[slot];
     if (!(cnt > 0.f)) return;
+    first = pl.s_start[slot]; last = pl.s_start[slot + 1];
     cden = fmaxf(cnt, El<T>::rnd(1e-6f));
     fresh = c.overwrite_on_insert && !pl.s_was[slot];
-    if (tid == 0) {
-      const int a0 = pl.s_start[slot], a1 = pl.s_start[slot + 1];
-      int nn = 0;
-      for (int a = a0; a < a1; ++a) {
-        const int t = pl.s_ord[a];
-        s_cand[nn] = p.cand[(long long)b * p.cand_bs + t]; s_wt[nn] = pl.s_w[t]; ++nn;
-      }
-      s_n = nn;
-    }
   }
-  __syncthreads();
-  const int nn = s_n;
+  // candidates a0 + 0..31 of the list in the lanes: a mask of those that count, their rows and weights
+  auto list_at = [&](int a0, int& ce, float& w) {
+    const int a = a0 + lane;
+    bool on = a < last;
+    ce = 0; w = 1.f;
+    if (on) {
+      if (exact) { on = (pl.e_flag[a] & 1) && pl.e_tgt[a] == slot; ce = p.cand[(long long)b * p.cand_bs + a]; }
+      else { ce = pl.s_ord[a]; w = pl.s_w[a]; }
+    }
+    return __ballot_sync(0xffffffffu, on);
+  };
   const int gslot = W + (exact ? 0 : Me) + slot;
+  T* const kbuf = (T*)p.st.k_buf + (long long)b * Hkv * Lbuf * Dh;
+  T* const vbuf = (T*)p.st.v_buf + (long long)b * Hkv * Lbuf * Dh;
   constexpr int R = 8;
-  const bool runs = (Dh % R) == 0;
-  for (int e0 = tid * R; e0 < HD; e0 += NT * R) {
-    const int h = e0 / Dh, d0 = e0 % Dh;
-    T* pk = kb + ((long long)h * Lbuf + gslot) * Dh + d0;
-    T* pv = vb + ((long long)h * Lbuf + gslot) * Dh + d0;
-    float ok[R], ov[R], ak[R], av[R];
-    if (runs) { load_run<T, R>(pk, ok); load_run<T, R>(pv, ov); }
-    else for (int i = 0; i < R; ++i) { ok[i] = (e0 + i < HD) ? El<T>::ld(kb + ((long long)((e0 + i) / Dh) * Lbuf + gslot) * Dh + (e0 + i) % Dh) : 0.f;
-                                       ov[i] = (e0 + i < HD) ? El<T>::ld(vb + ((long long)((e0 + i) / Dh) * Lbuf + gslot) * Dh + (e0 + i) % Dh) : 0.f; }
+  const bool runs = PACKED || (Dh % R) == 0;
+  const int nch = (HD + R - 1) / R;                                  // chunks of the K row, then as many of the V row
+  for (int x0 = 0; x0 < 2 * nch; x0 += GT) {
+    const int x = x0 + tid;
+    const bool isv = x >= nch;
+    const int e0 = (isv ? x - nch : x) * R, h = e0 / Dh, d0 = e0 % Dh;
+    // a chunk below the phase-safe half of a summary key is left alone
+    const bool live = x < 2 * nch && !(runs && !exact && !isv && d0 + R <= lf);
+    T* const buf = isv ? vbuf : kbuf;
+    const void* sblk = isv ? p.vblk : p.kblk;
+    const void* sbuf = isv ? p.st.v_buf : p.st.k_buf;
+    const long long sbs = isv ? p.vb_bs : p.kb_bs, srs = isv ? p.vb_rs : p.kb_rs;
+    auto at = [&](int e) { return buf + ((long long)(e / Dh) * Lbuf + gslot) * Dh + e % Dh; };
+    float old[R], acc[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) { ak[i] = 0.f; av[i] = 0.f; }
-    for (int q = 0; q < nn; ++q) {
-      const int ce = s_cand[q];
-      const float w = s_wt[q];
-      float xk[R], xv[R];
-      if (runs) {
-        load_run<T, R>(src_row<T>(p, p.st.k_buf, p.kblk, p.kb_bs, p.kb_rs, b, ce, h) + d0, xk);
-        load_run<T, R>(src_row<T>(p, p.st.v_buf, p.vblk, p.vb_bs, p.vb_rs, b, ce, h) + d0, xv);
-      } else {
-        for (int i = 0; i < R; ++i) {
-          const int hh = (e0 + i) / Dh, dd = (e0 + i) % Dh;
-          xk[i] = (e0 + i < HD) ? El<T>::ld(src_row<T>(p, p.st.k_buf, p.kblk, p.kb_bs, p.kb_rs, b, ce, hh) + dd) : 0.f;
-          xv[i] = (e0 + i < HD) ? El<T>::ld(src_row<T>(p, p.st.v_buf, p.vblk, p.vb_bs, p.vb_rs, b, ce, hh) + dd) : 0.f;
+    for (int i = 0; i < R; ++i) { old[i] = 0.f; acc[i] = 0.f; }
+    uint32_t oldw[R / 2], accw[R / 2];                               // (bf16 runs: the same, two elements a word)
+    if (PACKED && live) {
+      const uint4 t = *reinterpret_cast<const uint4*>(buf + ((long long)h * Lbuf + gslot) * Dh + d0);
+      oldw[0] = t.x; oldw[1] = t.y; oldw[2] = t.z; oldw[3] = t.w;
+      accw[0] = accw[1] = accw[2] = accw[3] = 0u;
+#pragma unroll
+      for (int i = 0; i < R / 2; ++i) { old[2 * i] = __uint_as_float(oldw[i] << 16); old[2 * i + 1] = __uint_as_float(oldw[i] & 0xffff0000u); }
+    } else if (live) {
+      if (runs) load_run<T, R>(buf + ((long long)h * Lbuf + gslot) * Dh + d0, old);
+      else for (int i = 0; i < R; ++i) if (e0 + i < HD) old[i] = El<T>::ld(at(e0 + i));
+    }
+    auto row_of = [&](int ce, float (&y)[R]) {
+      if (runs) { load_run<T, R>(src_row<T>(p, sbuf, sblk, sbs, srs, b, ce, h) + d0, y); return; }
+      for (int i = 0; i < R; ++i)
+        y[i] = e0 + i < HD ? El<T>::ld(src_row<T>(p, sbuf, sblk, sbs, srs, b, ce, (e0 + i) / Dh) + (e0 + i) % Dh) : 0.f;
+    };
+    for (int a0 = first; a0 < last; a0 += 32) {
+      int lce; float lw;
+      unsigned on = list_at(a0, lce, lw);
+      while (on != 0u) {
+        constexpr int NB = 4;
+        if constexpr (PACKED) {
+          uint4 y[NB];
+          uint32_t w2[NB];
+          bool have[NB];
+#pragma unroll
+          for (int q = 0; q < NB; ++q) {
+            have[q] = on != 0u;
+            const int src = have[q] ? __ffs(on) - 1 : 0;
+            on &= on - 1u;
+            const int ce = __shfl_sync(0xffffffffu, lce, src);
+            w2[q] = __float_as_uint(__shfl_sync(0xffffffffu, lw, src));      // a bf16 value: its word's upper half
+            w2[q] |= w2[q] >> 16;
+            if (have[q] && live) y[q] = *reinterpret_cast<const uint4*>(src_row<T>(p, sbuf, sblk, sbs, srs, b, ce, h) + d0);
+          }
+#pragma unroll
+          for (int q = 0; q < NB; ++q) {
+            if (!have[q] || !live) continue;
+            const uint32_t yw[4] = {y[q].x, y[q].y, y[q].z, y[q].w};
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i)
+              accw[i] = badd2(accw[i], exact ? badd2(yw[i], bneg2(oldw[i])) : bmul2(yw[i], w2[q]));
+          }
+        } else {
+          // one candidate at a time: single precision, unaligned rows, head sizes that are no multiple of a chunk
+          const int src = __ffs(on) - 1;
+          on &= on - 1u;
+          const int ce = __shfl_sync(0xffffffffu, lce, src);
+          const float w = __shfl_sync(0xffffffffu, lw, src);
+          if (live) {
+            float y[R];
+            row_of(ce, y);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+              if (exact) acc[i] = t_add<T>(acc[i], t_sub<T>(y[i], old[i]));
+              else acc[i] = t_add<T>(acc[i], t_mul<T>(y[i], w));
+            }
+          }
         }
       }
+    }
+    if (!live) continue;
+    if constexpr (PACKED) {
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        if (exact) { ak[i] = t_add<T>(ak[i], t_sub<T>(xk[i], ok[i])); av[i] = t_add<T>(av[i], t_sub<T>(xv[i], ov[i])); }
-        else { ak[i] = t_add<T>(ak[i], t_mul<T>(xk[i], w)); av[i] = t_add<T>(av[i], t_mul<T>(xv[i], w)); }
-      }
+      for (int i = 0; i < R / 2; ++i) { acc[2 * i] = __uint_as_float(accw[i] << 16); acc[2 * i + 1] = __uint_as_float(accw[i] & 0xffff0000u); }
     }
     // the slot's EMA rate depends on the head only: one sigmoid per run, not one per element
     const float eta_run = (exact || fresh) ? 1.f : t_sigmoid<T>(p.eta_logit[h]);
+    float nv[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int e = e0 + i;
-      if (e >= HD) break;
+      nv[i] = old[i];
+      if (e >= HD) continue;
       const int hh = runs ? h : e / Dh, dd = runs ? d0 + i : e % Dh;
-      T* qk = runs ? pk + i : kb + ((long long)hh * Lbuf + gslot) * Dh + dd;
-      T* qv = runs ? pv + i : vb + ((long long)hh * Lbuf + gslot) * Dh + dd;
       if (exact) {                                                     // mem + sum of deltas
-        El<T>::st(qk, t_add<T>(ok[i], ak[i]));
-        const float nv = t_add<T>(ov[i], av[i]);
-        El<T>::st(qv, nv);
-        stash[e] = nv;
+        nv[i] = t_add<T>(old[i], acc[i]);
+        if (isv) stash[e] = nv[i];
       } else {                                                         // phase-safe EMA
         const float eta = fresh ? 1.f : (runs ? eta_run : t_sigmoid<T>(p.eta_logit[hh]));
-        El<T>::st(qv, t_add<T>(ov[i], t_mul<T>(eta, t_sub<T>(t_div<T>(av[i], cden), ov[i]))));
-        if (dd >= lf) {
-          const float inc = El<T>::rnd(__fmul_rn(t_div<T>(ak[i], cden), c.energy_scale));
-          const float nk = t_add<T>(ok[i], t_mul<T>(eta, t_sub<T>(inc, ok[i])));
-          El<T>::st(qk, nk);
-          stash[hh * lfd + dd - lf] = nk;
+        if (isv) nv[i] = t_add<T>(old[i], t_mul<T>(eta, t_sub<T>(t_div<T>(acc[i], cden), old[i])));
+        else if (dd >= lf) {
+          const float inc = El<T>::rnd(__fmul_rn(t_div<T>(acc[i], cden), c.energy_scale));
+          nv[i] = t_add<T>(old[i], t_mul<T>(eta, t_sub<T>(inc, old[i])));
+          stash[hh * lfd + dd - lf] = nv[i];
         }
       }
     }
+    if (runs) store_run<T, R>(buf + ((long long)h * Lbuf + gslot) * Dh + d0, nv);
+    else
+      for (int i = 0; i < R; ++i)
+        if (e0 + i < HD) El<T>::st(at(e0 + i), nv[i]);
   }
-  if (tid == 0) al[gslot] = 1;
-  __syncthreads();
+  if (tid == 0) p.st.allowed[(long long)b * Lbuf + gslot] = 1;
+  if constexpr (WPS == 1) __syncwarp();
+  else if constexpr (WPS == 8) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"r"(1 + gid), "n"(GT) : "memory");     // (a group may have left)
   const int nn_norm = exact ? Dh : lfd;
   T* cachep = exact ? (T*)p.st.exact_v_norm + (long long)b * Hkv * Me * Dh : (T*)p.st.sum_lf_k_norm + (long long)b * Hkv * Ms * lfd;
   const int Mb = exact ? Me : Ms;
-  for (int h = warp; h < Hkv; h += NW) {
+  for (int h = tid >> 5; h < Hkv; h += WPS) {
     float ss = 0.f;
     for (int d = lane; d < nn_norm; d += 32) { const float v = stash[h * nn_norm + d]; ss += v * v; }
     const float den = fmaxf(El<T>::rnd(sqrtf(warp_sum(ss))), 1e-6f);
@@ -708,6 +788,26 @@ extern "C" int64_t coda_b200_route_scratch_bytes(const coda_layer_cfg* cfg) {
   return (int64_t)route_scratch_bytes(cfg);
 }
 
+// K and V rows of the state and of the block can be read and written as 16-byte vectors
+template <typename T>
+static int rows_vec16(const RouteParams& p) {
+  return (p.c.Dh * sizeof(T)) % 16 == 0 && ((uintptr_t)p.st.k_buf % 16 == 0) && ((uintptr_t)p.st.v_buf % 16 == 0) &&
+         ((uintptr_t)p.kblk % 16 == 0) && ((uintptr_t)p.vblk % 16 == 0) && (p.kb_rs * sizeof(T)) % 16 == 0 &&
+         (p.vb_rs * sizeof(T)) % 16 == 0 && (p.kb_bs * sizeof(T)) % 16 == 0 && (p.vb_bs * sizeof(T)) % 16 == 0;
+}
+
+template <typename T, bool PACKED>
+static void launch_apply(const RouteParams& p, int nslots, cudaStream_t s) {
+  const int HD = p.c.Hkv * p.c.Dh;
+  const size_t smem = sizeof(float) * (size_t)HD * (HD <= 128 ? 4 : HD <= 256 ? 2 : 1);
+  if (HD <= 128) route_apply_kernel<T, 1, PACKED><<<dim3((nslots + 3) / 4, p.c.B), 128, smem, s>>>(p, nslots);
+  else if (HD <= 256) route_apply_kernel<T, 2, PACKED><<<dim3((nslots + 1) / 2, p.c.B), 128, smem, s>>>(p, nslots);
+  else {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(route_apply_kernel<T, 8, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    route_apply_kernel<T, 8, PACKED><<<dim3(nslots, p.c.B), 256, smem, s>>>(p, nslots);
+  }
+}
+
 template <typename T>
 // phase 0: everything; 1: scores and decisions only (they read the state and write the scratch and the LRU
 // stamps: nothing the attention of the same block reads is touched); 2: slot updates and the ring rewrite only.
@@ -738,28 +838,27 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
       CODA_CHECK_LAUNCH("route_block (score)");
     }
     const int tmax = p.te > p.ts ? p.te : p.ts;
-    const size_t smem2 = 32 * (size_t)(c.Me > 0 ? c.Me : 1) + 4 * ((size_t)2 * (tmax + 1) + 4 * (size_t)(p.te + 1) + 4 * (size_t)(p.ts + 1) +
-                         3 * (size_t)(c.Ms + 1) + 2) + c.Me + c.Ms + 64;
+    const size_t me1 = c.Me > 0 ? c.Me : 1;
+    const size_t smem2 = me1 * (16 + 8 + 4 + 4 + 4) + 4 * ((size_t)2 * (tmax + 1) + 2 * (size_t)(p.te + 1) + 2 * (size_t)(p.ts + 1) +
+                         (size_t)c.Ms + 2) + c.Me + c.Ms + 64;
     CODA_REQUIRE(smem2 <= 200 * 1024, CODA_ERR_LIMIT, "route_block: decision stage needs %zu bytes of shared memory", smem2);
     if (smem2 > 48 * 1024) cudaFuncSetAttribute(route_decide_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    route_decide_kernel<T><<<c.B, 64, smem2, s>>>(p);
+    route_decide_kernel<T><<<c.B, RD_THREADS, smem2, s>>>(p);
     CODA_CHECK_LAUNCH("route_block (decide)");
   }
   if (phase == 1) return CODA_OK;
   if (p.te > 0 || p.ts > 0) {
     const int tmax = p.te > p.ts ? p.te : p.ts;
-    const size_t smem3 = sizeof(float) * (size_t)HD + 8 * (size_t)(tmax > 0 ? tmax : 1);   // new row + the slot's candidate list
-    CODA_REQUIRE(smem3 <= 200 * 1024, CODA_ERR_LIMIT, "route_block: Hkv*Dh = %d with %d candidates per block needs %zu bytes of shared memory", HD, tmax, smem3);
-    if (smem3 > 48 * 1024) cudaFuncSetAttribute(route_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-    const int nslots = (c.Me > 0 ? p.te : 0) + (p.ts > 0 ? c.Ms : 0);
+    const size_t most = sizeof(float) * (size_t)HD + 8 * (size_t)(tmax > 0 ? tmax : 1);
+    CODA_REQUIRE(most <= 200 * 1024, CODA_ERR_LIMIT, "route_block: Hkv*Dh = %d with %d candidates per block needs %zu bytes of shared memory", HD, tmax, most);
+    const int nslots = (c.Me > 0 ? p.te : 0) + (c.Ms > 0 && p.ts > 0 ? c.Ms : 0);
     if (nslots > 0) {
-      route_apply_kernel<T><<<dim3(nslots, c.B), 128, smem3, s>>>(p);
+      if constexpr (sizeof(T) == 2) { if (rows_vec16<T>(p)) launch_apply<T, true>(p, nslots, s); else launch_apply<T, false>(p, nslots, s); }
+      else launch_apply<T, false>(p, nslots, s);
       CODA_CHECK_LAUNCH("route_block (apply)");
     }
   }
-  const int vec16 = (c.Dh * sizeof(T)) % 16 == 0 && ((uintptr_t)p.st.k_buf % 16 == 0) && ((uintptr_t)p.st.v_buf % 16 == 0) &&
-                    ((uintptr_t)p.kblk % 16 == 0) && ((uintptr_t)p.vblk % 16 == 0) && (p.kb_rs * sizeof(T)) % 16 == 0 &&
-                    (p.vb_rs * sizeof(T)) % 16 == 0 && (p.kb_bs * sizeof(T)) % 16 == 0 && (p.vb_bs * sizeof(T)) % 16 == 0;
+  const int vec16 = rows_vec16<T>(p);
   ring_rewrite_kernel<T><<<dim3(2 * c.Hkv, c.B), 256, 0, s>>>(p, vec16);
   CODA_CHECK_LAUNCH("route_block (ring)");
   return CODA_OK;

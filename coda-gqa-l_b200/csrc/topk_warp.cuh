@@ -6,7 +6,8 @@
 // index a left stopper when its element does not go before the pivot, and a right stopper when the pivot does not
 // go before it; the serial pass swaps the k-th left stopper (ascending) with the k-th right stopper (descending) while
 // the former lies below the latter.  A warp finds both lists with ballots and prefix counts, 32 elements at a time, and
-// swaps all pairs at once.  Median, the at most 3-element tail, heap paths and the final sort of a few elements stay on one lane.
+// swaps all pairs at once.  Median, the at most 3-element tail, heap paths and the sort of more than 16
+// elements stay on one lane.
 #pragma once
 #include "topk_order.h"
 
@@ -47,6 +48,25 @@ __device__ __forceinline__ int partition_warp(It* q, int first, int last, const 
   return first + cut;
 }
 
+// sort_range of at most 16 elements [0, n): there it is a plain insertion sort, which is stable, so the place of an
+// element is the number of elements that go before it or tie with it from the left.  All lanes call.
+template <typename It, typename Cmp>
+__device__ __forceinline__ void sort_small_warp(It* q, int n, Cmp before) {
+  const int lane = threadIdx.x & 31;
+  It mine = q[0];
+  int place = 0;
+  if (lane < n) {
+    mine = q[lane];
+    for (int j = 0; j < n; ++j) {
+      const It o = q[j];
+      place += before(o, mine) || (j < lane && !before(mine, o)) ? 1 : 0;
+    }
+  }
+  __syncwarp();
+  if (lane < n) q[place] = mine;
+  __syncwarp();
+}
+
 // topk_queue by one warp; `scratch`: 2 * n uint16.  n < 65536.
 template <typename V, bool LARGEST>
 __device__ __forceinline__ void topk_queue_warp(Item<V>* q, int n, int k, bool sorted, uint16_t* scratch) {
@@ -75,10 +95,11 @@ __device__ __forceinline__ void topk_queue_warp(Item<V>* q, int n, int k, bool s
     if (lane == 0) {
       if (heap) { heap_select(q, first, nth + 1, last, before); swap_items(q, first, nth); }
       else insertion_sort(q, first, last, before);
-      if (sorted) sort_range(q, 0, k - 1, before);
+      if (sorted && k - 1 > 16) sort_range(q, 0, k - 1, before);
     }
   }
   __syncwarp();
+  if (sorted && k - 1 <= 16) sort_small_warp(q, k - 1, before);
 }
 
 }  // namespace topk_order

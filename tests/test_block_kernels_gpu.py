@@ -2,8 +2,9 @@
 import pytest
 import torch
 
-from tests.helpers import TOL_BF16, orc, rel_err
+from tests.helpers import SCENARIOS, TOL_BF16, orc, rel_err
 from tests.scenarios import randomize_weights
+from tests.test_parity_gpu import _run
 
 pytestmark = pytest.mark.gpu
 
@@ -72,6 +73,30 @@ def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
     y = stream(q) - d(lam).transpose(1, 2)[..., None] * stream(qn)
     y = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + mod.eps) * d(mod.head_norm.weight)
     assert rel_err(out, y.transpose(1, 2).reshape(B, Lq, H * Dh)) < 5e-6
+
+
+@pytest.mark.parametrize("kw,Te,Ts,block,B", [
+    # one warp per slot: more candidates than a warp has lanes, more than 16 LRU victims, slot counts that are not
+    # multiples of 32, one and several tiles of scores
+    (dict(num_heads=4, num_kv_heads=2, embed_dim=128, num_landmarks_exact=40, num_landmarks_summary=33), 40, 70, 96, 2),
+    (dict(num_heads=3, num_kv_heads=3, embed_dim=192, num_landmarks_exact=70, num_landmarks_summary=100), 33, 90, 100, 2),
+    (dict(num_heads=2, num_kv_heads=2, embed_dim=256, num_landmarks_exact=8, num_landmarks_summary=32), 8, 64, 48, 3),
+    # rows above 256 elements: four warps per slot; one KV head: no cluster
+    (dict(num_heads=8, num_kv_heads=8, embed_dim=512, num_landmarks_exact=12, num_landmarks_summary=1), 5, 64, 70, 1),
+    (dict(num_heads=2, num_kv_heads=1, embed_dim=128, num_landmarks_exact=1, num_landmarks_summary=3), 8, 64, 64, 2),
+    # head_dim 20 and 12: chunks that straddle heads and the phase-safe half
+    (dict(num_heads=4, num_kv_heads=2, embed_dim=80, num_landmarks_exact=16, num_landmarks_summary=16), 8, 64, 40, 2),
+    (dict(num_heads=4, num_kv_heads=4, embed_dim=48, num_landmarks_exact=5, num_landmarks_summary=7), 3, 9, 33, 2),
+])
+def test_block_routing_matches_oracle(monkeypatch, kw, Te, Ts, block, B):
+    """Scores, decisions, slot writes and events of the block write in fp32: occupancy, stamps and counters exactly, bank
+    contents and outputs to the parity tolerance."""
+    sc = dict(model=dict(window=32, exact_candidates_per_block=Te, summary_candidates_per_block=Ts, collect_metrics=True, **kw),
+              model_seed=7, state_seed=9, B=B, random_gate=True,
+              inputs=dict(kind="mixture", centroids=48, sigma=0.3, seed=11, L=4 * block + 40, Ldec=3),
+              phases=[("prefill", 0, 4 * block + 40, block), ("decode", 0, 3)])
+    monkeypatch.setitem(SCENARIOS, "block_routing", sc)
+    _run("block_routing", check_golden=False)
 
 
 @pytest.mark.parametrize("kw,B", [

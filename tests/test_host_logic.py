@@ -221,3 +221,15 @@ def test_captured_step_key_sees_every_way_a_parameter_can_change():
     assert stack._graph_key(list(states[:2]) + [SimpleNamespace(active_exact=4, active_summary=4)], torch.bfloat16) != k
     assert stack._graph_key(states, torch.float32) != k
     assert key() == k
+
+
+def test_quotient_of_bf16_values_rounds_the_same_from_an_approximate_reciprocal():
+    """The device code rounds a * (1 / b) instead of a / b to bf16: every pair of significands, the product perturbed by
+    twice the error it can have (a reciprocal good to an ulp and one rounding: below 2^-22), rounds as the quotient does."""
+    import torch
+    a = torch.arange(128, 256, dtype=torch.float64)[:, None]
+    b = torch.arange(128, 256, dtype=torch.float64)[None, :]
+    q = a / b
+    want = q.to(torch.float32).to(torch.bfloat16)
+    for eps in (-2.0 ** -21, 2.0 ** -21):
+        assert torch.equal((q * (1 + eps)).to(torch.float32).to(torch.bfloat16), want)
