@@ -189,122 +189,150 @@ __global__ void __launch_bounds__(256) route_score_kernel(RouteParams p) {
 // ---- the same scores with the KV heads side by side: one CTA per (bank, state, head), the heads of a state in one cluster ----
 // route_score_bank walks the heads one after the other (2 x Hkv tile loads per output tile, each a memory round
 // trip); here CTA h computes head h's rounded dot products only, leaves them in its shared memory, and after one
-// cluster barrier every CTA finishes the output rows r with r % Hkv == h: it adds the Hkv partials in head order
-// (the order route_score_bank adds them in, so the results are the same bits), takes the mean, applies the slot
+// cluster barrier every CTA finishes the output rows r with r % Hkv == h, a warp per row: it adds the Hkv partials in head
+// order (the order route_score_bank adds them in, so the results are the same bits), takes the mean, applies the slot
 // masks and keeps the running first-index argmax of its rows.
-template <typename T, int TM>
+// Bound: issue slots of many small CTAs (staging, the rounded division per element, the products), so the tile
+// follows the bank: ROWS candidates x COLS slots x KC elements with COLS = 32 where both banks have at most 32 slots,
+// and KC = 32 where the phase-safe half of a key has at most 32 elements.
+// Per block: 17 -> 12 us (64 states, 2 heads of 64, 64 slots a bank), 94 -> 54 us (512 states, 3 heads of 64, 32 slots),
+// 25.5 -> 24 us (32 states, 8 heads of 128, 64 slots).
+template <typename T, int ROWS, int COLS, int KC>
 __device__ __forceinline__ void route_score_bank_heads(const RouteParams& p, int b, bool exact, float* sm) {
-  constexpr int ROWS = 16 * TM;
+  constexpr int TX = COLS / 4, RG = 256 / TX;                 // threads along the columns (4 each) / row groups
+  constexpr int TM = ROWS > RG ? ROWS / RG : 1;               // rows per thread; row groups beyond ROWS only stage
   const coda_layer_cfg& c = p.c;
-  const int tid = threadIdx.x, h = blockIdx.z;
+  const int tid = threadIdx.x, h = blockIdx.z, lane = tid & 31, warp = tid >> 5;
   const int Hkv = c.Hkv, Dh = c.Dh, lf = Dh / 2, W = c.W, Me = c.Me, Ms = c.Ms;
   const int n = exact ? Dh : Dh - lf, M = exact ? Me : Ms, Tn = exact ? p.te : p.ts;
   const int active = exact ? c.active_exact : c.active_summary;
   const T* cache = exact ? (const T*)p.st.exact_v_norm + (long long)b * Hkv * Me * Dh
                          : (const T*)p.st.sum_lf_k_norm + (long long)b * Hkv * Ms * n;
   const uint8_t* al = p.st.allowed + (long long)b * (W + Me + Ms);
-  float* As = sm;                                  // [RS_KC][ROWS]
-  float* Bs = As + RS_KC * ROWS;                   // [RS_KC][RS_COLS]
-  float* Ps = Bs + RS_KC * RS_COLS;                // [ROWS][RS_COLS]   this head's rounded dots (read by the whole cluster)
-  float* Fs = Ps + ROWS * RS_COLS;                 // [ROWS / Hkv + 1][RS_COLS + 1]  final scores of the rows this CTA owns
-  float* den = Fs + (ROWS / Hkv + 1) * (RS_COLS + 1);   // [ROWS]
-  int* cidx = reinterpret_cast<int*>(den + ROWS);  // [ROWS]
-  const int ty = tid >> 4, tx = tid & 15;          // 16 x 16 thread grid
-  const int nown_max = ROWS / Hkv + 1;
+  float* As = sm;                                  // [KC][ROWS]
+  float* Bs = As + KC * ROWS;                      // [KC][COLS]
+  float* Ps = Bs + KC * COLS;                      // [ROWS][COLS]   this head's rounded dots (read by the whole cluster)
+  float* den = Ps + ROWS * COLS;                   // [ROWS]
+  float* rbest = den + ROWS;                       // [ROWS] running best score and slot of the rows this CTA owns
+  int* rbi = reinterpret_cast<int*>(rbest + ROWS);
+  int* cidx = rbi + ROWS;                          // [ROWS]
+  const int ty = tid / TX, tx = tid % TX;
+  const bool one_chunk = n <= KC;
 
   for (int r0 = 0; r0 < Tn; r0 += ROWS) {
     const int nrows = min(ROWS, Tn - r0);
     __syncthreads();
     for (int r = tid; r < ROWS; r += 256) cidx[r] = r < nrows ? p.cand[(long long)b * p.cand_bs + r0 + r] : -1;
     __syncthreads();
-    // ||x|| of every candidate of the tile for this head, batched loads  (memory_banks.py:498-500).  One thread per
-    // row (every fourth): the fp32 sum of squares runs over the elements in order, as route_score_bank's does.
-    {
-      const int r = tid >> 2, part = tid & 3;
+    auto row_at = [&](int r) {
+      return exact ? src_row<T>(p, p.st.v_buf, p.vblk, p.vb_bs, p.vb_rs, b, cidx[r], h)
+                   : src_row<T>(p, p.st.k_buf, p.kblk, p.kb_bs, p.kb_rs, b, cidx[r], h) + lf;
+    };
+    // ||x|| of every candidate of the tile for this head (memory_banks.py:498-500): the fp32 sum of squares runs over the
+    // elements in order, one thread per row, as route_score_bank's does.  Rows that one chunk holds are summed from
+    // shared memory below instead.
+    if (!one_chunk && tid < ROWS) {
       float ss = 0.f;
-      if (r < ROWS && cidx[r] >= 0) {
-        const T* row = exact ? src_row<T>(p, p.st.v_buf, p.vblk, p.vb_bs, p.vb_rs, b, cidx[r], h)
-                             : src_row<T>(p, p.st.k_buf, p.kblk, p.kb_bs, p.kb_rs, b, cidx[r], h) + lf;
-        if (part == 0) {
-          int d = 0;
-          for (; d + 16 <= n; d += 16) {
-            float x[16];
-            load_run<T, 16>(row + d, x);
+      if (cidx[tid] >= 0) {
+        const T* row = row_at(tid);
+        int d = 0;
+        for (; d + 16 <= n; d += 16) {
+          float x[16];
+          load_run<T, 16>(row + d, x);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) ss = fmaf(x[i], x[i], ss);
-          }
-          for (; d < n; ++d) { const float v = El<T>::ld(row + d); ss = fmaf(v, v, ss); }
+          for (int i = 0; i < 16; ++i) ss = fmaf(x[i], x[i], ss);
         }
+        for (; d < n; ++d) { const float v = El<T>::ld(row + d); ss = fmaf(v, v, ss); }
       }
-      if (r < ROWS && part == 0) den[r] = fmaxf(El<T>::rnd(sqrtf(ss)), 1e-6f);
+      den[tid] = fmaxf(El<T>::rnd(sqrtf(ss)), 1e-6f);
     }
-    float best = 0.f; int bi = 0;                  // running first-index argmax of owned row `tid` (tid < rows owned)
-    for (int c0 = 0; c0 < M; c0 += RS_COLS) {
+    for (int c0 = 0; c0 < M; c0 += COLS) {
       float acc[TM][4];
 #pragma unroll
       for (int i = 0; i < TM; ++i) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
-      for (int k0 = 0; k0 < n; k0 += RS_KC) {
+      for (int k0 = 0; k0 < n; k0 += KC) {
         __syncthreads();
-        {
-          constexpr int KRUN_A = RS_KC * ROWS / 256;          // 16 (64-row tile) or 4 (16-row tile)
-          const int r = tid % ROWS, kq0 = (tid / ROWS) * KRUN_A;
-          float x[KRUN_A];
+        // stage: candidates (normalised, dtype-rounded) and cache rows, both transposed to [k][row]; every thread owns a
+        // run of consecutive k of one row of each and loads it in one batch
+        constexpr int KRUN_A = KC * ROWS / 256, KRUN_B = KC * COLS / 256;
+        const int ar = tid % ROWS, ak = (tid / ROWS) * KRUN_A, bc = tid % COLS, bk = (tid / COLS) * KRUN_B;
+        float xa[KRUN_A], xb[KRUN_B];
 #pragma unroll
-          for (int i = 0; i < KRUN_A; ++i) x[i] = 0.f;
-          if (cidx[r] >= 0) {
-            const T* row = exact ? src_row<T>(p, p.st.v_buf, p.vblk, p.vb_bs, p.vb_rs, b, cidx[r], h)
-                                 : src_row<T>(p, p.st.k_buf, p.kblk, p.kb_bs, p.kb_rs, b, cidx[r], h) + lf;
-            if (k0 + kq0 + KRUN_A <= n) load_run<T, KRUN_A>(row + k0 + kq0, x);
-            else
-              for (int i = 0; i < KRUN_A; ++i) if (k0 + kq0 + i < n) x[i] = El<T>::ld(row + k0 + kq0 + i);
-            const float dn = den[r];
-#pragma unroll
-            for (int i = 0; i < KRUN_A; ++i) x[i] = t_div<T>(x[i], dn);
-          }
-#pragma unroll
-          for (int i = 0; i < KRUN_A; ++i) As[(kq0 + i) * ROWS + r] = x[i];
+        for (int i = 0; i < KRUN_B; ++i) xb[i] = 0.f;
+        if (c0 + bc < M) {
+          const T* row = cache + ((long long)h * M + c0 + bc) * n + k0 + bk;
+          if (k0 + bk + KRUN_B <= n) load_run<T, KRUN_B>(row, xb);
+          else
+            for (int i = 0; i < KRUN_B; ++i) if (k0 + bk + i < n) xb[i] = El<T>::ld(row + i);
         }
-        {
-          constexpr int KRUN_B = RS_KC * RS_COLS / 256;       // 16
-          const int col = tid % RS_COLS, kq0 = (tid / RS_COLS) * KRUN_B, m = c0 + col;
-          float x[KRUN_B];
 #pragma unroll
-          for (int i = 0; i < KRUN_B; ++i) x[i] = 0.f;
-          if (m < M) {
-            const T* row = cache + ((long long)h * M + m) * n;
-            if (k0 + kq0 + KRUN_B <= n) load_run<T, KRUN_B>(row + k0 + kq0, x);
-            else
-              for (int i = 0; i < KRUN_B; ++i) if (k0 + kq0 + i < n) x[i] = El<T>::ld(row + k0 + kq0 + i);
-          }
-#pragma unroll
-          for (int i = 0; i < KRUN_B; ++i) Bs[(kq0 + i) * RS_COLS + col] = x[i];
+        for (int i = 0; i < KRUN_A; ++i) xa[i] = 0.f;
+        const bool have = cidx[ar] >= 0;
+        if (have) {
+          const T* row = row_at(ar) + k0 + ak;
+          if (k0 + ak + KRUN_A <= n) load_run<T, KRUN_A>(row, xa);
+          else
+            for (int i = 0; i < KRUN_A; ++i) if (k0 + ak + i < n) xa[i] = El<T>::ld(row + i);
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < KRUN_B; ++i) Bs[(bk + i) * COLS + bc] = xb[i];
+        if (one_chunk && c0 == 0) {
+#pragma unroll
+          for (int i = 0; i < KRUN_A; ++i) As[(ak + i) * ROWS + ar] = xa[i];
+          __syncthreads();
+          if (tid < ROWS) {
+            float ss = 0.f;
 #pragma unroll 8
-        for (int kq = 0; kq < RS_KC; ++kq) {
-          float a[TM];
+            for (int d = 0; d < n; ++d) { const float v = As[d * ROWS + tid]; ss = fmaf(v, v, ss); }
+            den[tid] = fmaxf(El<T>::rnd(sqrtf(ss)), 1e-6f);
+          }
+          __syncthreads();
+        }
+        if (have) {
+          const float dn = den[ar];
 #pragma unroll
-          for (int i = 0; i < TM; ++i) a[i] = As[kq * ROWS + ty * TM + i];
-          const float4 bv = *reinterpret_cast<const float4*>(Bs + kq * RS_COLS + tx * 4);
+          for (int i = 0; i < KRUN_A; ++i) xa[i] = t_div<T>(xa[i], dn);
+        }
 #pragma unroll
-          for (int i = 0; i < TM; ++i) {
-            acc[i][0] = fmaf(a[i], bv.x, acc[i][0]); acc[i][1] = fmaf(a[i], bv.y, acc[i][1]);
-            acc[i][2] = fmaf(a[i], bv.z, acc[i][2]); acc[i][3] = fmaf(a[i], bv.w, acc[i][3]);
+        for (int i = 0; i < KRUN_A; ++i) As[(ak + i) * ROWS + ar] = xa[i];
+        __syncthreads();
+        if (ty < ROWS / TM) {
+          const int kend = min(KC, n - k0);
+#pragma unroll 8
+          for (int kq = 0; kq < kend; ++kq) {
+            float a[TM];
+            const float* ap = As + kq * ROWS + ty * TM;
+            if constexpr (TM == 4) { const float4 v = *reinterpret_cast<const float4*>(ap); a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w; }
+            else if constexpr (TM == 2) { const float2 v = *reinterpret_cast<const float2*>(ap); a[0] = v.x; a[1] = v.y; }
+            else a[0] = ap[0];
+            const float4 bv = *reinterpret_cast<const float4*>(Bs + kq * COLS + tx * 4);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+              acc[i][0] = fmaf(a[i], bv.x, acc[i][0]); acc[i][1] = fmaf(a[i], bv.y, acc[i][1]);
+              acc[i][2] = fmaf(a[i], bv.z, acc[i][2]); acc[i][3] = fmaf(a[i], bv.w, acc[i][3]);
+            }
           }
         }
       }
       // every CTA of the cluster has read the previous tile's partials before they are overwritten
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      __syncwarp();
+      if (r0 > 0 || c0 > 0) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (ty < ROWS / TM) {
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) Ps[(ty * TM + i) * RS_COLS + tx * 4 + jj] = El<T>::rnd(acc[i][jj]);
+        for (int i = 0; i < TM; ++i)
+          *reinterpret_cast<float4*>(Ps + (ty * TM + i) * COLS + tx * 4) =
+              make_float4(El<T>::rnd(acc[i][0]), El<T>::rnd(acc[i][1]), El<T>::rnd(acc[i][2]), El<T>::rnd(acc[i][3]));
+      }
+      __syncwarp();
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-      // rows r = h, h + Hkv, ... of the tile are finished here: partials of all heads, in head order
-      for (int o = tid; o < nown_max * RS_COLS; o += 256) {
-        const int lr = o / RS_COLS, col = o % RS_COLS, r = h + lr * Hkv;
-        if (r < ROWS) {
-          const uint32_t local = tma::smem_u32(Ps + r * RS_COLS + col);
+      // rows r = h, h + Hkv, ... of the tile are finished here, a warp per row: partials of all heads, in head order
+      for (int r = h + warp * Hkv; r < nrows; r += 8 * Hkv) {
+        float best = -INFINITY, first = 0.f;
+        int bi = 0x7fffffff;
+#pragma unroll
+        for (int cc = 0; cc < COLS / 32; ++cc) {
+          const int col = lane + 32 * cc, m = c0 + col;
+          const uint32_t local = tma::smem_u32(Ps + r * COLS + col);
           float pv[8];                                 // all requests first, then the sum in head order
 #pragma unroll
           for (int hh = 0; hh < 8; ++hh) {
@@ -318,43 +346,68 @@ __device__ __forceinline__ void route_score_bank_heads(const RouteParams& p, int
           float tot = 0.f;
 #pragma unroll
           for (int hh = 0; hh < 8; ++hh) if (hh < Hkv) tot += pv[hh];
-          const int m = c0 + col;
-          float sc = El<T>::rnd(tot / (float)Hkv);
-          if (m >= M) sc = -INFINITY;                                   // padding column: never wins
-          else if (m >= active || (exact && !al[W + m])) sc = -1e9f;    // (:646-650, :875-877)
-          Fs[lr * (RS_COLS + 1) + col] = sc;
-        }
-      }
-      __syncthreads();
-      {
-        const int r = h + tid * Hkv;                 // owned row `tid`
-        if (tid < nown_max && r < nrows) {
-          for (int col = 0; col < RS_COLS && c0 + col < M; ++col) {
-            const float sc = Fs[tid * (RS_COLS + 1) + col];
-            if ((c0 == 0 && col == 0) || sc > best) { best = sc; bi = c0 + col; }
+          if (m < M) {
+            float sc = El<T>::rnd(tot / (float)Hkv);
+            if (m >= active || (exact && !al[W + m])) sc = -1e9f;         // (:646-650, :875-877)
+            if (cc == 0) first = sc;
+            if (sc > best || bi == 0x7fffffff) { best = sc != sc ? -INFINITY : sc; bi = m; }
           }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        }
+        // a score that is not a number wins only from the very first slot, where the running maximum starts
+        if (lane == 0) {
+          if (c0 == 0) { const bool nan0 = first != first; rbest[r] = nan0 ? first : best; rbi[r] = nan0 ? 0 : bi; }
+          else if (best > rbest[r]) { rbest[r] = best; rbi[r] = bi; }
         }
       }
     }
-    {
-      const int r = h + tid * Hkv;
-      if (tid < nown_max && r < nrows) {
-        if (exact) { p.ex_best[(long long)b * c.Te + r0 + r] = best; p.ex_bi[(long long)b * c.Te + r0 + r] = bi; }
-        else p.su_idx[(long long)b * c.Ts + r0 + r] = bi;
+    __syncwarp();
+    if (lane == 0) {
+      for (int r = h + warp * Hkv; r < nrows; r += 8 * Hkv) {
+        if (exact) { p.ex_best[(long long)b * c.Te + r0 + r] = rbest[r]; p.ex_bi[(long long)b * c.Te + r0 + r] = rbi[r]; }
+        else p.su_idx[(long long)b * c.Ts + r0 + r] = rbi[r];
       }
     }
   }
   // no CTA may leave while another still reads its partials
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) route_score_heads_kernel(RouteParams p) {
-  extern __shared__ float sm[];
+template <int COLS, int KCS>
+constexpr size_t route_score_heads_floats() {
+  const size_t e = (size_t)RS_KC * 16 + RS_KC * COLS + 16 * COLS + 4 * 16, s = (size_t)KCS * 64 + KCS * COLS + 64 * COLS + 4 * 64;
+  return e > s ? e : s;
+}
+
+template <typename T, int COLS, int KCS>
+__global__ void __launch_bounds__(256, 4) route_score_heads_kernel(RouteParams p) {
+  extern __shared__ __align__(16) float sm[];
   const bool exact = blockIdx.x == 0;
   // (both branches are uniform over a cluster: its CTAs differ in blockIdx.z only)
-  if (exact) { if (p.te > 0 && p.c.Me > 0) route_score_bank_heads<T, 1>(p, blockIdx.y, true, sm); }
-  else if (p.ts > 0 && p.c.Ms > 0) route_score_bank_heads<T, 4>(p, blockIdx.y, false, sm);
+  if (exact) { if (p.te > 0 && p.c.Me > 0) route_score_bank_heads<T, 16, COLS, RS_KC>(p, blockIdx.y, true, sm); }
+  else if (p.ts > 0 && p.c.Ms > 0) route_score_bank_heads<T, 64, COLS, KCS>(p, blockIdx.y, false, sm);
+}
+
+template <typename T, int COLS, int KCS>
+static cudaError_t launch_score_heads(const RouteParams& p, cudaStream_t s) {
+  const size_t smem = sizeof(float) * route_score_heads_floats<COLS, KCS>();
+  if (smem > 48 * 1024) cudaFuncSetAttribute(route_score_heads_kernel<T, COLS, KCS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(2, p.c.B, p.c.Hkv);
+  lc.blockDim = dim3(256, 1, 1);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = p.c.Hkv;
+  lc.attrs = at; lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, route_score_heads_kernel<T, COLS, KCS>, p);
 }
 
 // Per-state plan written by route_decide and consumed by route_apply (all int32 / fp32, in global scratch).
@@ -820,18 +873,9 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
     if (smem1 > 48 * 1024) cudaFuncSetAttribute(route_score_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
     if (c.Hkv >= 2 && c.Hkv <= 8 && c.B <= 65535) {
       // the heads of a state side by side: clusters of Hkv CTAs along z
-      const size_t smemh = sizeof(float) * (size_t)(RS_KC * 64 + RS_KC * RS_COLS + 64 * RS_COLS + (64 / c.Hkv + 1) * (RS_COLS + 1) + 64 + 64);
-      if (smemh > 48 * 1024) cudaFuncSetAttribute(route_score_heads_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemh);
-      cudaLaunchConfig_t lc = {};
-      lc.gridDim = dim3(2, c.B, c.Hkv);
-      lc.blockDim = dim3(256, 1, 1);
-      lc.dynamicSmemBytes = smemh;
-      lc.stream = s;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = c.Hkv;
-      lc.attrs = at; lc.numAttrs = 1;
-      cudaError_t e = cudaLaunchKernelEx(&lc, route_score_heads_kernel<T>, p);
+      const bool narrow = c.Me <= 32 && c.Ms <= 32, low = c.Dh - c.Dh / 2 <= 32;
+      const cudaError_t e = narrow ? (low ? launch_score_heads<T, 32, 32>(p, s) : launch_score_heads<T, 32, 64>(p, s))
+                                   : (low ? launch_score_heads<T, 64, 32>(p, s) : launch_score_heads<T, 64, 64>(p, s));
       if (e != cudaSuccess) { coda_set_error("route_block (score): %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
     } else {
       route_score_kernel<T><<<dim3(2, c.B), 256, smem1, s>>>(p);
