@@ -718,19 +718,19 @@ int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, DecodeParams p, 
   constexpr int BUDGET = 226 * 1024;
   // as many ring stages as fit beside the fixed buffers (at least 2, at most DA_MAX_STAGES)
   const int fixed = DecodeSmem<DH>(0, p.G, p.Lbuf).total + 1024;
-  int stages = (BUDGET / da_ctas(DH, NQ) - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES);
-  const int ctas = stages >= 2 ? da_ctas(DH, NQ) : 1;      // (long masks: the ring takes what one CTA per SM has)
-  if (stages < 2) stages = (BUDGET - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES);
-  if (stages > DA_MAX_STAGES) stages = DA_MAX_STAGES;
-  stages &= ~1;                                      // even: each ring stage belongs to one consumer group (see the kernel)
-  CODA_REQUIRE(stages >= 2, CODA_ERR_LIMIT, "decode_attend: %d slots leave no room for the tile ring in shared memory", p.Lbuf);
-  p.stages = stages;
-  const size_t smem = (size_t)DecodeSmem<DH>(stages, p.G, p.Lbuf).total + 1024;
   static coda_device_once once;
   const int num_sms = coda_on_first_use(once, [] {
     cudaFuncSetAttribute(decode_attend_kernel<DH, NQ, APPEND>, cudaFuncAttributeMaxDynamicSharedMemorySize, BUDGET);
   });
   const int nplanes = p.B * p.Hkv;
+  // (no more planes than SMs, or a ring that half an SM cannot hold: one CTA per SM takes the whole budget)
+  const int ctas = nplanes > num_sms && (BUDGET / da_ctas(DH, NQ) - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES) >= 2 ? da_ctas(DH, NQ) : 1;
+  int stages = (BUDGET / ctas - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES);
+  if (stages > DA_MAX_STAGES) stages = DA_MAX_STAGES;
+  stages &= ~1;                                      // even: each ring stage belongs to one consumer group (see the kernel)
+  CODA_REQUIRE(stages >= 2, CODA_ERR_LIMIT, "decode_attend: %d slots leave no room for the tile ring in shared memory", p.Lbuf);
+  p.stages = stages;
+  const size_t smem = (size_t)DecodeSmem<DH>(stages, p.G, p.Lbuf).total + 1024;
   // Programmatic dependent launch: the CTAs may start (shared-memory carve-up, barrier initialisation) while the
   // kernel before this one on the stream is still finishing; they wait for it (griddepcontrol.wait) before the
   // first global access.
