@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
     cp_commit();
   };
 
+  grid_chain();
   unsigned bits = 0u;
   int t = next_tile(warp, bits);
   if (t < ntiles) { load(Ks, KS, kbase, kblk, p.kb_rs, t); load(Vs, DH, vbase, vblk, p.vb_rs, t); }
@@ -264,7 +265,7 @@ int launch(const AttnParams& p, cudaStream_t s) {
   constexpr int bytes = Lay::FLOATS * 4;
   static coda_device_once once;
   coda_on_first_use(once, [] { cudaFuncSetAttribute(attend_f32_kernel<DH, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
-  attend_f32_kernel<DH, TM><<<dim3((p.Lq + Lay::BQ - 1) / Lay::BQ, p.H, p.B), AF_WARPS * 32, bytes, s>>>(p);
+  coda_launch_chained(attend_f32_kernel<DH, TM>, dim3((p.Lq + Lay::BQ - 1) / Lay::BQ, p.H, p.B), dim3(AF_WARPS * 32), bytes, s, 1, p);
   CODA_CHECK_LAUNCH("attend (f32)");
   return CODA_OK;
 }

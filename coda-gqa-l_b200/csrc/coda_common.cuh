@@ -177,6 +177,28 @@ void coda_set_error(const char* fmt, ...);
 #define CODA_CHECK_LAUNCH(what) do { cudaError_t e__ = cudaGetLastError(); if (e__ != cudaSuccess) { \
   coda_set_error("%s: %s", what, cudaGetErrorString(e__)); return CODA_ERR_LAUNCH; } } while (0)
 
+// ---- chained launches ----------------------------------------------------------------------------
+// The kernels of a prefill block follow one another on a stream, a few microseconds each, and the gap between two
+// launches is one to two.  Launched this way a kernel may be brought onto the SMs while the one before it finishes; it
+// calls grid_chain() before its first global access (writes too), which holds it back until that kernel has
+// completed and lets the next one come.  A 2048-token prefill of 64 states (8 blocks of 5 launches): 1512 -> 1420 us.
+__device__ __forceinline__ void grid_chain() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t coda_launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster_z, Args&&... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid; lc.blockDim = block; lc.dynamicSmemBytes = smem; lc.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = (unsigned)cluster_z;
+  lc.attrs = at; lc.numAttrs = cluster_z > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...);
+}
+
 // ---- per-device launch set-up ------------------------------------------------------------------
 // cudaFuncSetAttribute and the SM count belong to a device, not to the process: a process that drives several
 // GPUs (a model spread over devices, one thread per GPU) repeats them for every device it launches on.

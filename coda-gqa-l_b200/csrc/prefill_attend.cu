@@ -218,6 +218,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         tma::mbar_init(&v_full[i], 1); tma::mbar_init(&v_empty[i], 1);
       }
       tma::fence_barrier_init();
+      grid_chain();
       tma::mbar_expect_tx(q_full, Q_BYTES);         // (the barriers are this thread's own so far: Q may leave at once)
 #pragma unroll
       for (int hf = 0; hf < HALVES; ++hf) {
@@ -230,6 +231,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     tc_fence_before();
   } else if (warp == 0) {                            // visibility of the prefix slots; tiles with no visible slot drop out
+    grid_chain();
     const uint8_t* al = p.allowed + (long long)b * p.Lbuf;
     int nv = 0;
     for (int j0 = 0; j0 < NP; j0 += 4) {
@@ -322,6 +324,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     }
   } else {
     // =========================== softmax / correction / epilogue ===========================
+    grid_chain();                                         // (lambda and the output rows are this role's)
     const int s = warp >> 1;                              // 0 = signal rows, 1 = noise rows
     const int row = (warp & 1) * 32 + lane;               // row of the query tile
     const int grow = r0 + row;                            // row inside the block
@@ -544,7 +547,7 @@ int launch_prefill(const CUtensorMap* maps, const PrefillParams& p, cudaStream_t
     cudaFuncSetAttribute(prefill_attend_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
   });
   dim3 grid((p.blk + PF_BM - 1) / PF_BM, p.H, p.B);
-  prefill_attend_kernel<DH><<<grid, PF_THREADS, smem, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
+  coda_launch_chained(prefill_attend_kernel<DH>, grid, dim3(PF_THREADS), smem, s, 1, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
   CODA_CHECK_LAUNCH("prefill_attend");
   return CODA_OK;
 }

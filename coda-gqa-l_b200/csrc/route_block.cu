@@ -181,6 +181,7 @@ __device__ __forceinline__ void route_score_bank(const RouteParams& p, int b, bo
 template <typename T>
 __global__ void __launch_bounds__(256) route_score_kernel(RouteParams p) {
   extern __shared__ float sm[];
+  grid_chain();
   const bool exact = blockIdx.x == 0;
   if (exact) { if (p.te > 0 && p.c.Me > 0) route_score_bank<T, 1>(p, blockIdx.y, true, sm); }
   else if (p.ts > 0 && p.c.Ms > 0) route_score_bank<T, 4>(p, blockIdx.y, false, sm);
@@ -388,6 +389,7 @@ constexpr size_t route_score_heads_floats() {
 template <typename T, int COLS, int KCS>
 __global__ void __launch_bounds__(256, 4) route_score_heads_kernel(RouteParams p) {
   extern __shared__ __align__(16) float sm[];
+  grid_chain();
   const bool exact = blockIdx.x == 0;
   // (both branches are uniform over a cluster: its CTAs differ in blockIdx.z only)
   if (exact) { if (p.te > 0 && p.c.Me > 0) route_score_bank_heads<T, 16, COLS, RS_KC>(p, blockIdx.y, true, sm); }
@@ -398,16 +400,7 @@ template <typename T, int COLS, int KCS>
 static cudaError_t launch_score_heads(const RouteParams& p, cudaStream_t s) {
   const size_t smem = sizeof(float) * route_score_heads_floats<COLS, KCS>();
   if (smem > 48 * 1024) cudaFuncSetAttribute(route_score_heads_kernel<T, COLS, KCS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(2, p.c.B, p.c.Hkv);
-  lc.blockDim = dim3(256, 1, 1);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = p.c.Hkv;
-  lc.attrs = at; lc.numAttrs = 1;
-  return cudaLaunchKernelEx(&lc, route_score_heads_kernel<T, COLS, KCS>, p);
+  return coda_launch_chained(route_score_heads_kernel<T, COLS, KCS>, dim3(2, p.c.B, p.c.Hkv), dim3(256), smem, s, p.c.Hkv, p);
 }
 
 // Per-state plan written by route_decide and consumed by route_apply (all int32 / fp32, in global scratch).
@@ -463,6 +456,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
   long long* last = (long long*)p.st.mem_last_exact + (long long)b * Me;
   Plan pl = plan_of(p, b);
   const int Ae = c.active_exact;
+  grid_chain();
   for (int t = tid; t < tmax; t += NT) {
     const int e = p.cand[(long long)b * p.cand_bs + t];
     c_e[t] = e;
@@ -607,6 +601,7 @@ __global__ void __launch_bounds__(WPS == 8 ? 256 : 128, WPS == 8 ? 3 : 6) route_
   constexpr int GT = 32 * WPS, GROUPS = (WPS == 8 ? 256 : 128) / GT; // threads of a slot's group, groups per CTA
   const int b = blockIdx.y, lane = threadIdx.x & 31, gid = threadIdx.x / GT, tid = threadIdx.x % GT;
   const int job = blockIdx.x * GROUPS + gid;
+  grid_chain();
   if (job >= nslots) return;
   const int Hkv = c.Hkv, Dh = c.Dh, HD = Hkv * Dh, lf = Dh / 2, lfd = Dh - lf;
   float* stash = stash_all + gid * HD;
@@ -810,6 +805,7 @@ __global__ void __launch_bounds__(256) ring_rewrite_kernel(RouteParams p, int ve
   T* ring = (T*)(pass ? p.st.v_buf : p.st.k_buf) + ((long long)b * c.Hkv + h) * Lbuf * Dh;
   const T* src = (const T*)(pass ? p.vblk : p.kblk) + (long long)b * (pass ? p.vb_bs : p.kb_bs) + (long long)h * Dh;
   const long long rs = pass ? p.vb_rs : p.kb_rs;
+  grid_chain();
   if (vec16) ring_plane<T, uint4>(ring, src, rs, Dh, drop, kept, bstart, nnew, tid, NT);
   else ring_plane<T, T>(ring, src, rs, Dh, drop, kept, bstart, nnew, tid, NT);
   if (blockIdx.x == 0) {
@@ -853,11 +849,11 @@ template <typename T, bool PACKED>
 static void launch_apply(const RouteParams& p, int nslots, cudaStream_t s) {
   const int HD = p.c.Hkv * p.c.Dh;
   const size_t smem = sizeof(float) * (size_t)HD * (HD <= 128 ? 4 : HD <= 256 ? 2 : 1);
-  if (HD <= 128) route_apply_kernel<T, 1, PACKED><<<dim3((nslots + 3) / 4, p.c.B), 128, smem, s>>>(p, nslots);
-  else if (HD <= 256) route_apply_kernel<T, 2, PACKED><<<dim3((nslots + 1) / 2, p.c.B), 128, smem, s>>>(p, nslots);
+  if (HD <= 128) coda_launch_chained(route_apply_kernel<T, 1, PACKED>, dim3((nslots + 3) / 4, p.c.B), dim3(128), smem, s, 1, p, nslots);
+  else if (HD <= 256) coda_launch_chained(route_apply_kernel<T, 2, PACKED>, dim3((nslots + 1) / 2, p.c.B), dim3(128), smem, s, 1, p, nslots);
   else {
     if (smem > 48 * 1024) cudaFuncSetAttribute(route_apply_kernel<T, 8, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    route_apply_kernel<T, 8, PACKED><<<dim3(nslots, p.c.B), 256, smem, s>>>(p, nslots);
+    coda_launch_chained(route_apply_kernel<T, 8, PACKED>, dim3(nslots, p.c.B), dim3(256), smem, s, 1, p, nslots);
   }
 }
 
@@ -878,7 +874,7 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
                                    : (low ? launch_score_heads<T, 64, 32>(p, s) : launch_score_heads<T, 64, 64>(p, s));
       if (e != cudaSuccess) { coda_set_error("route_block (score): %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
     } else {
-      route_score_kernel<T><<<dim3(2, c.B), 256, smem1, s>>>(p);
+      coda_launch_chained(route_score_kernel<T>, dim3(2, c.B), dim3(256), smem1, s, 1, p);
       CODA_CHECK_LAUNCH("route_block (score)");
     }
     const int tmax = p.te > p.ts ? p.te : p.ts;
@@ -887,7 +883,7 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
                          (size_t)c.Ms + 2) + c.Me + c.Ms + 64;
     CODA_REQUIRE(smem2 <= 200 * 1024, CODA_ERR_LIMIT, "route_block: decision stage needs %zu bytes of shared memory", smem2);
     if (smem2 > 48 * 1024) cudaFuncSetAttribute(route_decide_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    route_decide_kernel<T><<<c.B, RD_THREADS, smem2, s>>>(p);
+    coda_launch_chained(route_decide_kernel<T>, dim3(c.B), dim3(RD_THREADS), smem2, s, 1, p);
     CODA_CHECK_LAUNCH("route_block (decide)");
   }
   if (phase == 1) return CODA_OK;
@@ -903,7 +899,7 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
     }
   }
   const int vec16 = rows_vec16<T>(p);
-  ring_rewrite_kernel<T><<<dim3(2 * c.Hkv, c.B), 256, 0, s>>>(p, vec16);
+  coda_launch_chained(ring_rewrite_kernel<T>, dim3(2 * c.Hkv, c.B), dim3(256), 0, s, 1, p, vec16);
   CODA_CHECK_LAUNCH("route_block (ring)");
   return CODA_OK;
 }
