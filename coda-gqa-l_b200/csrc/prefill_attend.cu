@@ -28,7 +28,7 @@ constexpr int PF_BN = 64;        // keys per tile
 constexpr int PF_M = 128;        // MMA rows
 constexpr int PF_THREADS = 192;  // warps 0-3: softmax, 4: TMA, 5: MMA issuer
 constexpr int PF_TMEM_COLS = 256;
-constexpr int pf_stages(int dh) { return dh == 128 ? 2 : 3; }   // K tiles (and V tiles) in flight; two CTAs fit an SM
+constexpr int PF_STAGES = 2;     // K tiles (and V tiles) in flight
 constexpr float PF_RESCALE_GAP = 8.0f;   // log2 units the running max may lag before O is rescaled
 
 struct PrefillParams {
@@ -95,6 +95,13 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// True in one lane of the (converged) warp, always the same one
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(pred));
+  return pred != 0;
+}
 
 // Shared-memory matrix descriptor, 128-byte swizzle, version 1 (Blackwell).  K-major operands (rows of 64
 // bf16 = 128 bytes, 8-row groups 1024 bytes apart): lbo unused (1), sbo = 1024.  MN-major operands (rows are
@@ -173,7 +180,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                       const __grid_constant__ CUtensorMap kpmap, const __grid_constant__ CUtensorMap vpmap,
                       const __grid_constant__ CUtensorMap kbmap, const __grid_constant__ CUtensorMap vbmap,
                       PrefillParams p) {
-  constexpr int STAGES = pf_stages(DH);
+  constexpr int STAGES = PF_STAGES;
   constexpr int HALVES = DH / 64;                 // 64-element (128-byte) column groups per row
   constexpr int Q_HALF = PF_M * 128;              // bytes of one column group of the stacked Q tile
   constexpr int Q_BYTES = HALVES * Q_HALF;
@@ -190,14 +197,12 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   unsigned char* sV = sK + STAGES * KV_BYTES;      // [STAGES][KV_BYTES]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + STAGES * KV_BYTES);
   uint64_t* q_full = bars;                          // 1
-  uint64_t* pv_done = bars + 1;                     // [buffer]
-  uint64_t* s_full = bars + 3;                      // [buffer]
-  uint64_t* p_full = bars + 5;                      // [buffer]
-  uint64_t* k_full = bars + 7;                      // [stage]
-  uint64_t* k_empty = k_full + STAGES;
-  uint64_t* v_full = k_empty + STAGES;
-  uint64_t* v_empty = v_full + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + STAGES);   // TMEM base, then the number of prefix tiles
+  uint64_t* s_full = bars + 1;                      // [buffer] S complete; K tile n sits in stage n % 2 = buffer, so: K stage free
+  uint64_t* p_full = bars + 3;                      // [buffer]
+  uint64_t* k_full = bars + 5;                      // [stage]
+  uint64_t* v_full = bars + 7;                      // [stage]
+  uint64_t* v_empty = bars + 9;                     // [stage] P.V complete: V stage free, O quiescent
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);   // TMEM base, then the number of prefix tiles
   uint32_t* sMask = tmem_slot + 2;                  // [NP][2] visibility bits of the n-th tile that is read
   const int NP = (p.Lbuf + PF_BN - 1) / PF_BN;      // prefix tiles
   unsigned short* sTile = reinterpret_cast<unsigned short*>(sMask + 2 * NP);   // [NP] which tile that is
@@ -208,30 +213,37 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 
   __shared__ int s_abort;                          // set by the first bounded wait of this CTA that expires
   int* const abortw = &s_abort;
+  // one K (or V) tile, the it-th that is read, into its stage
+  auto load_tile = [&](int it, int nv, const CUtensorMap* pm, const CUtensorMap* bm, unsigned char* ring, uint64_t* full) {
+    const int st = it % STAGES;
+    tma::mbar_expect_tx(&full[st], KV_BYTES);
+    unsigned char* dst = ring + st * KV_BYTES;
+#pragma unroll
+    for (int hf = 0; hf < HALVES; ++hf) {
+      if (it < nv) tma_load_3d(dst + hf * KV_HALF, pm, &full[st], hf * 64, (int)sTile[it] * PF_BN, b * p.Hkv + hk);
+      else tma_load_4d(dst + hf * KV_HALF, bm, &full[st], hf * 64, hk, p.t0 + (it - nv) * PF_BN, b);
+    }
+  };
   if (warp == 4) {
     if (lane == 0) {
       s_abort = 0;
       tma::mbar_init(q_full, 1);
-      for (int i = 0; i < 2; ++i) { tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], 4); tma::mbar_init(&pv_done[i], 1); }
-      for (int i = 0; i < STAGES; ++i) {
-        tma::mbar_init(&k_full[i], 1); tma::mbar_init(&k_empty[i], 1);
-        tma::mbar_init(&v_full[i], 1); tma::mbar_init(&v_empty[i], 1);
+      for (int i = 0; i < 2; ++i) {
+        tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], 4);
+        tma::mbar_init(&k_full[i], 1); tma::mbar_init(&v_full[i], 1); tma::mbar_init(&v_empty[i], 1);
       }
       tma::fence_barrier_init();
-      grid_chain();
-      tma::mbar_expect_tx(q_full, Q_BYTES);         // (the barriers are this thread's own so far: Q may leave at once)
+    }
+    grid_chain();
+    if (lane == 0) {                                 // (the barriers are this thread's own so far: Q may leave at once)
+      tma::mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll
       for (int hf = 0; hf < HALVES; ++hf) {
         tma_load_4d(sQ + hf * Q_HALF, &qmap, q_full, hf * 64, h, p.t0 + r0, b);
         tma_load_4d(sQ + hf * Q_HALF + PF_BM * 128, &qnmap, q_full, hf * 64, h, p.t0 + r0, b);
       }
     }
-  } else if (warp == 5) {                            // TMEM: half of the SM's columns, owned by the MMA warp
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(PF_TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    tc_fence_before();
-  } else if (warp == 0) {                            // visibility of the prefix slots; tiles with no visible slot drop out
-    grid_chain();
+    // visibility of the prefix slots; tiles with no visible slot drop out
     const uint8_t* al = p.allowed + (long long)b * p.Lbuf;
     int nv = 0;
     for (int j0 = 0; j0 < NP; j0 += 4) {
@@ -250,7 +262,16 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         }
       }
     }
-    if (lane == 0) tmem_slot[1] = (uint32_t)nv;
+    if (lane == 0) {
+      tmem_slot[1] = (uint32_t)nv;
+      load_tile(0, nv, &kpmap, &kbmap, sK, k_full);
+      if (nv + r0 / PF_BN + 1 > 1) load_tile(1, nv, &kpmap, &kbmap, sK, k_full);
+      load_tile(0, nv, &vpmap, &vbmap, sV, v_full);
+    }
+  } else if (warp == 5) {                            // TMEM: half of the SM's columns, owned by the MMA warp
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(PF_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    tc_fence_before();
   }
   __syncthreads();
   tc_fence_after();
@@ -260,67 +281,58 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 
   if (warp == 4) {
     // =========================== TMA producer ===========================
+    // K tile it needs Q.K^T it-2 to be done, long before V tile it needs P.V it-2: K runs one tile ahead
     if (lane == 0) {
-      auto load_tile = [&](int it, const CUtensorMap* pm, const CUtensorMap* bm, unsigned char* ring, uint64_t* full, uint64_t* empty, int code) {
-        const int st = it % STAGES;
-        if (it >= STAGES) tma::mbar_wait(&empty[st], ((it / STAGES) - 1) & 1, p.status, code, abortw);
-        tma::mbar_expect_tx(&full[st], KV_BYTES);
-        unsigned char* dst = ring + st * KV_BYTES;
-#pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) {
-          if (it < NV) tma_load_3d(dst + hf * KV_HALF, pm, &full[st], hf * 64, (int)sTile[it] * PF_BN, b * p.Hkv + hk);
-          else tma_load_4d(dst + hf * KV_HALF, bm, &full[st], hf * 64, hk, p.t0 + (it - NV) * PF_BN, b);
+      for (int it = 1; it < NT; ++it) {
+        if (it + 1 < NT) {
+          tma::mbar_wait(&s_full[(it + 1) & 1], ((it - 1) >> 1) & 1, p.status, 11, abortw);
+          load_tile(it + 1, NV, &kpmap, &kbmap, sK, k_full);
         }
-      };
-      // K runs one tile ahead of V: its stage is free as soon as Q.K^T is done, long before P.V
-      load_tile(0, &kpmap, &kbmap, sK, k_full, k_empty, 11);
-      for (int it = 0; it < NT; ++it) {
-        if (it + 1 < NT) load_tile(it + 1, &kpmap, &kbmap, sK, k_full, k_empty, 11);
-        load_tile(it, &vpmap, &vbmap, sV, v_full, v_empty, 15);
+        if (it >= 2) tma::mbar_wait(&v_empty[it & 1], ((it - 2) >> 1) & 1, p.status, 15, abortw);
+        load_tile(it, NV, &vpmap, &vbmap, sV, v_full);
       }
     }
   } else if (warp == 5) {
     // =========================== MMA issuer ===========================
-    if (lane == 0) {
-      constexpr uint32_t IDESC_QK = instr_desc(PF_BN, false);
-      constexpr uint32_t IDESC_PV = instr_desc(DH, true);
-      const uint32_t qbase = smem_u32(sQ);
-      // S = Q . K^T into buffer it & 1 (free: the P.V two tiles back, which read P from it, was issued earlier by
-      // this same thread and the tensor pipe executes in order)
-      auto issue_qk = [&](int it) {
-        const int st = it % STAGES;
-        tma::mbar_wait(&k_full[st], (it / STAGES) & 1, p.status, 14, abortw);
-        tc_fence_after();
-        const uint32_t kbase = smem_u32(sK + st * KV_BYTES);
-        const uint32_t dcol = tmem + (uint32_t)(it & 1) * PF_BN;
+    // The whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers that way.  Under
+    // a lane == 0 branch they are moved there one by one, some 100 cycles per MMA (430 + 790 cycles for a tile's P.V and
+    // Q.K^T), and the issue becomes the longest chain of the tile.
+    constexpr uint32_t IDESC_QK = instr_desc(PF_BN, false);
+    constexpr uint32_t IDESC_PV = instr_desc(DH, true);
+    const uint64_t qdesc = smem_desc(smem_u32(sQ), 16, 1024), kdesc = smem_desc(smem_u32(sK), 16, 1024);
+    const uint64_t vdesc = smem_desc(smem_u32(sV), KV_HALF, 1024);
+    // S = Q . K^T into buffer it & 1 (free: the P.V two tiles back, which read P from it, was issued earlier by
+    // this same lane and the tensor pipe executes in order)
+    auto issue_qk = [&](int it) {
+      tma::mbar_wait(&k_full[it & 1], (it >> 1) & 1, p.status, 14, abortw);
+      tc_fence_after();
+      const uint64_t kd = kdesc + (uint32_t)(it & 1) * (KV_BYTES >> 4);
+      const uint32_t dcol = tmem + (uint32_t)(it & 1) * PF_BN;
+      if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < KSTEPS_QK; ++kk) {
-          const uint64_t ad = smem_desc(qbase + (kk >> 2) * Q_HALF + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = smem_desc(kbase + (kk >> 2) * KV_HALF + (kk & 3) * 32, 16, 1024);
-          tc_mma(dcol, ad, bd, IDESC_QK, kk > 0 ? 1u : 0u);
-        }
+        for (int kk = 0; kk < KSTEPS_QK; ++kk)
+          tc_mma(dcol, qdesc + (((kk >> 2) * Q_HALF + (kk & 3) * 32) >> 4), kd + (((kk >> 2) * KV_HALF + (kk & 3) * 32) >> 4), IDESC_QK, kk > 0 ? 1u : 0u);
         tc_commit(&s_full[it & 1]);
-        tc_commit(&k_empty[st]);
-      };
-      tma::mbar_wait(q_full, 0, p.status, 13, abortw);
-      issue_qk(0);
-      if (NT > 1) issue_qk(1);
-      for (int it = 0; it < NT; ++it) {
-        const int st = it % STAGES;
-        tma::mbar_wait(&v_full[st], (it / STAGES) & 1, p.status, 17, abortw);
-        tma::mbar_wait(&p_full[it & 1], (it >> 1) & 1, p.status, 12, abortw);
-        tc_fence_after();
-        const uint32_t vbase = smem_u32(sV + st * KV_BYTES);
-        const uint32_t pcol = tmem + (uint32_t)(it & 1) * PF_BN;      // P (bf16 pairs) sits in the first 32 columns of S
-#pragma unroll
-        for (int kk = 0; kk < KSTEPS_PV; ++kk) {
-          const uint64_t bd = smem_desc(vbase + kk * 2048, KV_HALF, 1024);
-          tc_mma_ts(tmem + TM_O, pcol + kk * 8, bd, IDESC_PV, (it > 0 || kk > 0) ? 1u : 0u);
-        }
-        tc_commit(&pv_done[it & 1]);
-        tc_commit(&v_empty[st]);
-        if (it + 2 < NT) issue_qk(it + 2);
       }
+      __syncwarp();
+    };
+    tma::mbar_wait(q_full, 0, p.status, 13, abortw);
+    issue_qk(0);
+    if (NT > 1) issue_qk(1);
+    for (int it = 0; it < NT; ++it) {
+      tma::mbar_wait(&v_full[it & 1], (it >> 1) & 1, p.status, 17, abortw);
+      tma::mbar_wait(&p_full[it & 1], (it >> 1) & 1, p.status, 12, abortw);
+      tc_fence_after();
+      const uint64_t vd = vdesc + (uint32_t)(it & 1) * (KV_BYTES >> 4);
+      const uint32_t pcol = tmem + (uint32_t)(it & 1) * PF_BN;      // P (bf16 pairs) sits in the first 32 columns of S
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < KSTEPS_PV; ++kk)
+          tc_mma_ts(tmem + TM_O, pcol + kk * 8, vd + ((kk * 2048) >> 4), IDESC_PV, (it > 0 || kk > 0) ? 1u : 0u);
+        tc_commit(&v_empty[it & 1]);
+      }
+      __syncwarp();
+      if (it + 2 < NT) issue_qk(it + 2);
     }
   } else {
     // =========================== softmax / correction / epilogue ===========================
@@ -391,11 +403,11 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         l *= alpha;
       }
       // Rescale O when some row of this warp moved its exponent base (not for the first tile: the first P.V
-      // overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V.  (A barrier per
-      // buffer: s_full of tile it was committed behind P.V it-2, so the barrier of P.V it-1 is at most one phase
-      // behind and its parity is not ambiguous; the same holds for the last P.V in the epilogue.)
+      // overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V.  (s_full of
+      // tile it was committed behind P.V it-2, so the barrier of P.V it-1 is at most one phase behind and its parity is
+      // not ambiguous; the same holds for the last P.V in the epilogue.)
       if (__any_sync(0xffffffffu, (alpha != 1.f) && it > 0)) {
-        tma::mbar_wait(&pv_done[(it - 1) & 1], ((it - 1) >> 1) & 1, p.status, 19, abortw);
+        tma::mbar_wait(&v_empty[(it - 1) & 1], ((it - 1) >> 1) & 1, p.status, 19, abortw);
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < DH / 16; ++c) {
@@ -456,7 +468,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     float lam = 0.f;
     if (valid) lam = bf16_round(p.lam[(long long)b * p.lam_bs + (long long)(p.t0 + grow) * p.lam_rs + h]);
     constexpr int HC = DH / 2;                             // columns per thread
-    tma::mbar_wait(&pv_done[(NT - 1) & 1], ((NT - 1) >> 1) & 1, p.status, 18, abortw);
+    tma::mbar_wait(&v_empty[(NT - 1) & 1], ((NT - 1) >> 1) & 1, p.status, 18, abortw);
     tc_fence_after();
     const float inv = l > 0.f ? 1.f / l : 0.f;
     constexpr int XM = HC / 4 - 1;                         // chunks of 4 floats per exchanged row, minus one
@@ -534,8 +546,8 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 template <int DH>
 size_t prefill_smem(int Lbuf) {
   const int NP = (Lbuf + PF_BN - 1) / PF_BN;
-  return (size_t)(DH / 64) * PF_M * 128 + 2 * pf_stages(DH) * (size_t)(DH / 64) * PF_BN * 128 +
-         (7 + 4 * pf_stages(DH)) * 8 + 8 + (size_t)NP * 10 + 1024 + 16;
+  return (size_t)(DH / 64) * PF_M * 128 + 2 * PF_STAGES * (size_t)(DH / 64) * PF_BN * 128 +
+         11 * 8 + 8 + (size_t)NP * 10 + 1024 + 16;
 }
 
 template <int DH>
