@@ -26,7 +26,8 @@ namespace {
 constexpr int PF_BM = 64;        // query rows per CTA (each present twice: signal and noise)
 constexpr int PF_BN = 64;        // keys per tile
 constexpr int PF_M = 128;        // MMA rows
-constexpr int PF_THREADS = 192;  // warps 0-3: softmax, 4: TMA, 5: MMA issuer
+constexpr int PF_SWARPS = 8;     // softmax warps: two per 32 rows, each with half of a tile's keys
+constexpr int PF_THREADS = (PF_SWARPS + 2) * 32;  // warps 0-7: softmax, 8: TMA, 9: MMA issuer
 constexpr int PF_TMEM_COLS = 256;
 constexpr int PF_STAGES = 2;     // K tiles (and V tiles) in flight
 constexpr float PF_RESCALE_GAP = 8.0f;   // log2 units the running max may lag before O is rescaled
@@ -168,7 +169,15 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-__device__ __forceinline__ void bar_softmax_all() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void bar_softmax_all() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The two warps that share 32 rows (barrier 2 + rows / 32): a rendezvous, and one that tells whether `mine` held anywhere
+__device__ __forceinline__ void bar_pair(int rows32) { asm volatile("bar.sync %0, 64;" ::"r"(2 + rows32) : "memory"); }
+__device__ __forceinline__ bool bar_pair_any(int rows32, bool mine) {
+  uint32_t r;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %2, 0;\nbar.red.or.pred p, %1, 64, q;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(r) : "r"(2 + rows32), "r"(mine ? 1u : 0u) : "memory");
+  return r != 0;
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -203,7 +212,8 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   uint64_t* v_full = bars + 7;                      // [stage]
   uint64_t* v_empty = bars + 9;                     // [stage] P.V complete: V stage free, O quiescent
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);   // TMEM base, then the number of prefix tiles
-  uint32_t* sMask = tmem_slot + 2;                  // [NP][2] visibility bits of the n-th tile that is read
+  float* sMax = reinterpret_cast<float*>(tmem_slot + 2);   // [2][128] row maxima of the two halves of a tile, when a base may move
+  uint32_t* sMask = tmem_slot + 2 + 2 * PF_M;             // [NP][2] visibility bits of the n-th tile that is read
   const int NP = (p.Lbuf + PF_BN - 1) / PF_BN;      // prefix tiles
   unsigned short* sTile = reinterpret_cast<unsigned short*>(sMask + 2 * NP);   // [NP] which tile that is
 
@@ -224,12 +234,12 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       else tma_load_4d(dst + hf * KV_HALF, bm, &full[st], hf * 64, hk, p.t0 + (it - nv) * PF_BN, b);
     }
   };
-  if (warp == 4) {
+  if (warp == PF_SWARPS) {
     if (lane == 0) {
       s_abort = 0;
       tma::mbar_init(q_full, 1);
       for (int i = 0; i < 2; ++i) {
-        tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], 4);
+        tma::mbar_init(&s_full[i], 1); tma::mbar_init(&p_full[i], PF_SWARPS);
         tma::mbar_init(&k_full[i], 1); tma::mbar_init(&v_full[i], 1); tma::mbar_init(&v_empty[i], 1);
       }
       tma::fence_barrier_init();
@@ -268,7 +278,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       if (nv + r0 / PF_BN + 1 > 1) load_tile(1, nv, &kpmap, &kbmap, sK, k_full);
       load_tile(0, nv, &vpmap, &vbmap, sV, v_full);
     }
-  } else if (warp == 5) {                            // TMEM: half of the SM's columns, owned by the MMA warp
+  } else if (warp == PF_SWARPS + 1) {                // TMEM: half of the SM's columns, owned by the MMA warp
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(PF_TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     tc_fence_before();
@@ -279,7 +289,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   const int NV = (int)tmem_slot[1];                  // prefix tiles that are read
   const int NT = NV + r0 / PF_BN + 1;                // ... and the block tiles up to the diagonal
 
-  if (warp == 4) {
+  if (warp == PF_SWARPS) {
     // =========================== TMA producer ===========================
     // K tile it needs Q.K^T it-2 to be done, long before V tile it needs P.V it-2: K runs one tile ahead
     if (lane == 0) {
@@ -292,7 +302,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         load_tile(it, NV, &vpmap, &vbmap, sV, v_full);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == PF_SWARPS + 1) {
     // =========================== MMA issuer ===========================
     // The whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers that way.  Under
     // a lane == 0 branch they are moved there one by one, some 100 cycles per MMA (430 + 790 cycles for a tile's P.V and
@@ -337,118 +347,108 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   } else {
     // =========================== softmax / correction / epilogue ===========================
     grid_chain();                                         // (lambda and the output rows are this role's)
-    const int s = warp >> 1;                              // 0 = signal rows, 1 = noise rows
-    const int row = (warp & 1) * 32 + lane;               // row of the query tile
+    const int quarter = warp & 3;                         // TMEM lanes this warp may touch: 32 * quarter ..
+    const int hf = warp >> 2;                             // keys 32 * hf .. of every tile
+    const int s = quarter >> 1;                           // 0 = signal rows, 1 = noise rows
+    const int row = (quarter & 1) * 32 + lane;            // row of the query tile
     const int grow = r0 + row;                            // row inside the block
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint32_t o_col = lane_addr + TM_O;
 
-    float mb = -INFINITY;                                 // exponent base (lags the true max by < GAP)
-    float l = 0.f;
+    float mb = -INFINITY;                                 // exponent base (lags the true max by < GAP), the same in both halves
+    float l = 0.f;                                        // sum over this warp's keys
     for (int it = 0; it < NT; ++it) {
       const uint32_t s_col = lane_addr + (uint32_t)(it & 1) * PF_BN;
-      // Visibility per group of 32 keys.  cls: 2 = all visible, 0 = none, 1 = mixed; the class is the same for
+      // Visibility of this warp's 32 keys.  cls: 2 = all visible, 0 = none, 1 = mixed; the class is the same for
       // every lane of a warp: prefix slots carry one mask per state, and in a block tile the 32 rows of a warp
       // meet the causal diagonal inside one group only.
-      uint32_t vis[2]; int cls[2];
+      uint32_t vis; int cls;
       if (it < NV) {
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          vis[g] = sMask[2 * it + g];
-          cls[g] = vis[g] == 0xffffffffu ? 2 : (vis[g] == 0u ? 0 : 1);
-        }
+        vis = sMask[2 * it + hf];
+        cls = vis == 0xffffffffu ? 2 : (vis == 0u ? 0 : 1);
       } else {
-        const int c0 = (it - NV) * PF_BN;
+        const int c0 = (it - NV) * PF_BN + 32 * hf;
         const int nvis = grow - c0 + 1;                   // key c0+i visible iff c0+i <= grow
-        const int gd = (r0 + (warp & 1) * 32 - c0) >> 5;  // group holding this warp's diagonal
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const int nq = nvis - 32 * g;
-          vis[g] = nq >= 32 ? 0xffffffffu : (nq <= 0 ? 0u : ((1u << nq) - 1u));
-          cls[g] = g < gd ? 2 : (g == gd ? 1 : 0);
-        }
+        const int gd = (r0 + (quarter & 1) * 32 - c0) >> 5;       // 0: this group holds the warp's diagonal
+        vis = nvis >= 32 ? 0xffffffffu : (nvis <= 0 ? 0u : ((1u << nvis) - 1u));
+        cls = gd > 0 ? 2 : (gd == 0 ? 1 : 0);
       }
       tma::mbar_wait(&s_full[it & 1], (it >> 1) & 1, p.status, 16, abortw);
       tc_fence_after();
-      // S is read from TMEM once, all 64 keys of the row into registers; groups without a visible key are not read
-      uint32_t v[2][32];
-#pragma unroll
-      for (int g = 0; g < 2; ++g) if (cls[g] != 0) tc_ld32(s_col + g * 32, v[g]);
+      uint32_t v[32];
+      tc_ld32(s_col + hf * 32, v);
       tc_wait_ld();
       // row maximum over the visible keys
-      float mx = -INFINITY;
+      float m0 = -INFINITY, m1 = -INFINITY;
+      if (cls == 2) {
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        float m0 = -INFINITY, m1 = -INFINITY;
-        if (cls[g] == 2) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            m0 = max3(m0, __uint_as_float(v[g][i]), __uint_as_float(v[g][i + 1]));
-            m1 = max3(m1, __uint_as_float(v[g][i + 2]), __uint_as_float(v[g][i + 3]));
-          }
-        } else if (cls[g] == 1) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (!((vis[g] >> i) & 1u)) v[g][i] = 0xff800000u;       // -inf: exp gives 0 below
-            m0 = fmaxf(m0, __uint_as_float(v[g][i]));
-          }
+        for (int i = 0; i < 32; i += 4) {
+          m0 = max3(m0, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+          m1 = max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
         }
-        mx = max3(mx, m0, m1);
+      } else if (cls == 1) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (!((vis >> i) & 1u)) v[i] = 0xff800000u;     // -inf: exp gives 0 below
+          m0 = fmaxf(m0, __uint_as_float(v[i]));
+        }
       }
-      mx *= p.scale_log2;                                  // scale > 0: max commutes with the scaling
-      float alpha = 1.f;
-      if (mx > mb + PF_RESCALE_GAP || (mb == -INFINITY && mx > -INFINITY)) {
-        alpha = (mb == -INFINITY) ? 0.f : exp2f(mb - mx);
-        mb = mx;
-        l *= alpha;
-      }
-      // Rescale O when some row of this warp moved its exponent base (not for the first tile: the first P.V
-      // overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V.  (s_full of
-      // tile it was committed behind P.V it-2, so the barrier of P.V it-1 is at most one phase behind and its parity is
-      // not ambiguous; the same holds for the last P.V in the epilogue.)
-      if (__any_sync(0xffffffffu, (alpha != 1.f) && it > 0)) {
-        tma::mbar_wait(&v_empty[(it - 1) & 1], ((it - 1) >> 1) & 1, p.status, 19, abortw);
-        tc_fence_after();
+      float mx = fmaxf(m0, m1) * p.scale_log2;            // scale > 0: max commutes with the scaling
+      // The other half of the row is in another warp.  Most tiles move no base: one barrier says so for the 32 rows (and
+      // that both warps hold their part of S in registers, which P may then overwrite); else the maxima are exchanged.
+      if (bar_pair_any(quarter, mx > mb + PF_RESCALE_GAP || (mb == -INFINITY && mx > -INFINITY))) {
+        sMax[hf * PF_M + quarter * 32 + lane] = mx;
+        bar_pair(quarter);
+        mx = fmaxf(mx, sMax[(1 - hf) * PF_M + quarter * 32 + lane]);
+        float alpha = 1.f;
+        if (mx > mb + PF_RESCALE_GAP || (mb == -INFINITY && mx > -INFINITY)) {
+          alpha = (mb == -INFINITY) ? 0.f : exp2f(mb - mx);
+          mb = mx;
+          l *= alpha;
+        }
+        // Rescale O, each warp half of its columns, when some row moved its exponent base (not for the first tile: the
+        // first P.V overwrites O instead of accumulating); O must be quiescent: wait for the previous P.V.  (s_full of
+        // tile it was committed behind P.V it-2, so the barrier of P.V it-1 is at most one phase behind and its parity is
+        // not ambiguous; the same holds for the last P.V in the epilogue.)
+        if (it > 0) {
+          tma::mbar_wait(&v_empty[(it - 1) & 1], ((it - 1) >> 1) & 1, p.status, 19, abortw);
+          tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < DH / 16; ++c) {
-          uint32_t o[16];
-          tc_ld16(o_col + c * 16, o);
-          tc_wait_ld();
+          for (int c = hf * (DH / 32); c < (hf + 1) * (DH / 32); ++c) {
+            uint32_t o[16];
+            tc_ld16(o_col + c * 16, o);
+            tc_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tc_st16(o_col + c * 16, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tc_st16(o_col + c * 16, o);
+          }
         }
       }
-      // probabilities, written back over S as packed bf16 (key 2i, 2i+1 -> column i); every S column has been
-      // read by now
+      // probabilities, written back over S as packed bf16 (key 2i, 2i+1 -> column i)
       const float nref = mb == -INFINITY ? 0.f : -mb;
       const uint64_t scale2 = pk64(p.scale_log2, p.scale_log2), nref2 = pk64(nref, nref);
-      uint64_t sum0 = 0ull, sum1 = 0ull, sum2 = 0ull, sum3 = 0ull;     // four independent chains of packed pairs
+      uint64_t sum0 = 0ull, sum1 = 0ull;                  // independent chains of packed pairs
+      uint32_t pk[16];
+      if (cls == 0) {
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t pk[16];
-        if (cls[g] == 0) {
+        for (int i = 0; i < 16; ++i) pk[i] = 0u;
+      } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) pk[i] = 0u;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            // exponent arguments of two keys per instruction; two pairs in three on the special-function
-            // unit, the third on the FMA pipe
-            float x0, x1, a0, a1;
-            unpk64(fma2(pk64(__uint_as_float(v[g][2 * i]), __uint_as_float(v[g][2 * i + 1])), scale2, nref2), x0, x1);
-            if (i % 3 == 2) { ex2_poly2(x0, x1, a0, a1); } else { a0 = ex2_mufu(x0); a1 = ex2_mufu(x1); }
-            const uint64_t pr = pk64(a0, a1);
-            if ((i & 3) == 0) sum0 = add2(sum0, pr); else if ((i & 3) == 1) sum1 = add2(sum1, pr);
-            else if ((i & 3) == 2) sum2 = add2(sum2, pr); else sum3 = add2(sum3, pr);
-            pk[i] = pack2(a0, a1);
-          }
+        for (int i = 0; i < 16; ++i) {
+          // exponent arguments of two keys per instruction; two pairs in three on the special-function
+          // unit, the third on the FMA pipe
+          float x0, x1, a0, a1;
+          unpk64(fma2(pk64(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), scale2, nref2), x0, x1);
+          if (i % 3 == 2) { ex2_poly2(x0, x1, a0, a1); } else { a0 = ex2_mufu(x0); a1 = ex2_mufu(x1); }
+          const uint64_t pr = pk64(a0, a1);
+          if (i & 1) sum1 = add2(sum1, pr); else sum0 = add2(sum0, pr);
+          pk[i] = pack2(a0, a1);
         }
-        tc_st16(s_col + g * 16, pk);
       }
+      tc_st16(s_col + hf * 16, pk);
       {
         float t0, t1;
-        unpk64(add2(add2(sum0, sum1), add2(sum2, sum3)), t0, t1);
+        unpk64(add2(sum0, sum1), t0, t1);
         l += t0 + t1;
       }
       tc_wait_st();
@@ -458,78 +458,86 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     }
 
     // ---- epilogue: signal / l_s - lambda * noise / l_n, head RMSNorm, store ----
-    // The two streams of a query row sit 64 TMEM lanes apart, in different warps.  Each thread hands one half of its
-    // normalised columns to its partner (signal rows finish columns 0 .. Dh/2-1, noise rows the rest) through the
-    // shared memory of the query tile, which is dead once every Q.K^T has completed; partial sums of squares go
-    // through the K ring and the rounded rows through the V ring, so that a warp stores whole rows.  16-byte chunks
-    // are XORed with the row so that neither the row-wise writes nor the reads collide in a bank.
-    // fp32 end to end with a single rounding of the result.
+    // The two streams of a query row sit 64 TMEM lanes apart.  A thread finishes one quarter of the columns of its query
+    // (signal rows the lower half, noise rows the upper, each warp of the pair half of that) and hands the quarter its
+    // partner in the other stream finishes, normalised, through the shared memory of the query tile, which is dead once
+    // every Q.K^T has completed; row sums and partial sums of squares go through the K ring and the rounded rows
+    // through the V ring, so that a warp stores whole rows.  16-byte chunks are XORed with the row so that neither the
+    // row-wise writes nor the reads collide in a bank.  fp32 end to end with a single rounding of the result.
     const bool valid = grow < p.blk;
     float lam = 0.f;
     if (valid) lam = bf16_round(p.lam[(long long)b * p.lam_bs + (long long)(p.t0 + grow) * p.lam_rs + h]);
-    constexpr int HC = DH / 2;                             // columns per thread
+    constexpr int HC = DH / 2, HQ = DH / 4;                // columns per stream, per thread
     tma::mbar_wait(&v_empty[(NT - 1) & 1], ((NT - 1) >> 1) & 1, p.status, 18, abortw);
     tc_fence_after();
+    float* xl = reinterpret_cast<float*>(sK);              // [2][128] row sums of the halves
+    float* xsq = xl + 2 * PF_M;                            // [4][64] partial sums of squares
+    xl[hf * PF_M + quarter * 32 + lane] = l;
+    bar_pair(quarter);
+    l += xl[(1 - hf) * PF_M + quarter * 32 + lane];
     const float inv = l > 0.f ? 1.f / l : 0.f;
     constexpr int XM = HC / 4 - 1;                         // chunks of 4 floats per exchanged row, minus one
     float4* xown = reinterpret_cast<float4*>(sQ) + (size_t)(s * PF_BM + row) * (HC / 4);
     const float4* xpart = reinterpret_cast<const float4*>(sQ) + (size_t)((1 - s) * PF_BM + row) * (HC / 4);
-#pragma unroll
-    for (int c = 0; c < HC / 32; ++c) {
-      uint32_t o[32];
-      tc_ld32(o_col + (1 - s) * HC + c * 32, o);
+    auto load_o = [&](int col, uint32_t (&o)[HQ]) {
+      if constexpr (HQ == 32) tc_ld32(o_col + col, o); else tc_ld16(o_col + col, o);
       tc_wait_ld();
+    };
+    {
+      uint32_t o[HQ];
+      load_o((1 - s) * HC + hf * HQ, o);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        xown[(c * 8 + i) ^ (row & XM)] = make_float4(__uint_as_float(o[4 * i]) * inv, __uint_as_float(o[4 * i + 1]) * inv,
-                                                    __uint_as_float(o[4 * i + 2]) * inv, __uint_as_float(o[4 * i + 3]) * inv);
+      for (int i = 0; i < HQ / 4; ++i)
+        xown[(hf * (HQ / 4) + i) ^ (row & XM)] = make_float4(__uint_as_float(o[4 * i]) * inv, __uint_as_float(o[4 * i + 1]) * inv,
+                                                             __uint_as_float(o[4 * i + 2]) * inv, __uint_as_float(o[4 * i + 3]) * inv);
     }
     bar_softmax_all();
-    float dv[HC];                                          // sig - lam * noise of this thread's columns
+    float dv[HQ];                                          // sig - lam * noise of this thread's columns
     float sq = 0.f;
+    {
+      uint32_t o[HQ];
+      load_o(s * HC + hf * HQ, o);
 #pragma unroll
-    for (int c = 0; c < HC / 32; ++c) {
-      uint32_t o[32];
-      tc_ld32(o_col + s * HC + c * 32, o);
-      tc_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 x = xpart[(c * 8 + i) ^ (row & XM)];
+      for (int i = 0; i < HQ / 4; ++i) {
+        const float4 x = xpart[(hf * (HQ / 4) + i) ^ (row & XM)];
         const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float own = __uint_as_float(o[4 * i + e]) * inv;
           const float d = s == 0 ? fmaf(-lam, xv[e], own) : fmaf(-lam, own, xv[e]);
           sq = fmaf(d, d, sq);
-          dv[c * 32 + 4 * i + e] = d;
+          dv[4 * i + e] = d;
         }
       }
     }
-    float* xsq = reinterpret_cast<float*>(sK);             // [2][64] partial sums of squares
-    xsq[s * PF_BM + row] = sq;
-    if (p.norm_full) bar_softmax_all();
-    const float rs = p.norm_full ? rsqrtf((xsq[row] + xsq[PF_BM + row]) / (float)DH + p.eps) : 1.f;
+    float rs = 1.f;
+    if (p.norm_full) {
+      xsq[(s * 2 + hf) * PF_BM + row] = sq;
+      bar_softmax_all();
+      rs = rsqrtf(((xsq[row] + xsq[PF_BM + row]) + (xsq[2 * PF_BM + row] + xsq[3 * PF_BM + row])) / (float)DH + p.eps);
+    }
     constexpr int RC = DH / 8;                             // 16-byte chunks per output row
     uint4* srow = reinterpret_cast<uint4*>(sV) + (size_t)row * RC;
+    const int cbase = (s * 2 + hf) * HQ;                   // first of this thread's columns
 #pragma unroll
-    for (int i = 0; i < HC / 8; ++i) {
+    for (int i = 0; i < HQ / 8; ++i) {
       uint32_t w[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         float y0 = dv[8 * i + 2 * e] * rs, y1 = dv[8 * i + 2 * e + 1] * rs;
         if (p.norm_full) {
-          const __nv_bfloat162 wv = reinterpret_cast<const __nv_bfloat162*>(p.norm_w)[(s * HC) / 2 + 4 * i + e];
+          const __nv_bfloat162 wv = reinterpret_cast<const __nv_bfloat162*>(p.norm_w)[cbase / 2 + 4 * i + e];
           y0 *= __low2float(wv); y1 *= __high2float(wv);
         }
         w[e] = pack2(y0, y1);
       }
-      srow[(s * (HC / 8) + i) ^ (row & (RC - 1))] = make_uint4(w[0], w[1], w[2], w[3]);
+      srow[(cbase / 8 + i) ^ (row & (RC - 1))] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     bar_softmax_all();
     bf16* ob = p.out + (long long)b * p.out_bs + (long long)(p.t0 + r0) * p.out_rs + (long long)h * DH;
 #pragma unroll
-    for (int i = 0; i < PF_BM * RC / 128; ++i) {
-      const int x = i * 128 + tid, rr = x / RC, cc = x % RC;
+    for (int i = 0; i < PF_BM * RC / (32 * PF_SWARPS); ++i) {
+      const int x = i * 32 * PF_SWARPS + tid, rr = x / RC, cc = x % RC;
       if (r0 + rr < p.blk)
         *reinterpret_cast<uint4*>(ob + (long long)rr * p.out_rs + cc * 8) = reinterpret_cast<const uint4*>(sV)[rr * RC + (cc ^ (rr & (RC - 1)))];
     }
@@ -537,7 +545,7 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   }
 
   __syncthreads();                                     // every role meets here once all tensor work is done
-  if (warp == 5) {
+  if (warp == PF_SWARPS + 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(PF_TMEM_COLS) : "memory");
   }
@@ -547,7 +555,7 @@ template <int DH>
 size_t prefill_smem(int Lbuf) {
   const int NP = (Lbuf + PF_BN - 1) / PF_BN;
   return (size_t)(DH / 64) * PF_M * 128 + 2 * PF_STAGES * (size_t)(DH / 64) * PF_BN * 128 +
-         11 * 8 + 8 + (size_t)NP * 10 + 1024 + 16;
+         11 * 8 + 8 + 2 * PF_M * 4 + (size_t)NP * 10 + 1024 + 16;
 }
 
 template <int DH>
