@@ -20,7 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _lib
-from ._lib import LayerCfg, RingPos, StatePtrs, check, lib
+from ._lib import LayerCfg, RingPos, StatePtrs, StepLayer, check, lib
 from .primitives import HeadwiseRMSNorm, RotaryEmbedding
 from .state import CoDAGQALandmarkStatePerf2, allocate_state
 
@@ -611,10 +611,29 @@ class CoDAGQALandmarkPerf2(nn.Module):
                  off_gate=(H * Dh + 2 * Hkv * Dh + H) * es, gated=self.write_policy != "none",
                  inv_freq=inv_freq.data_ptr(), cos=cos_t.data_ptr(), sin=sin_t.data_ptr(), eta=eta.data_ptr(), nw=_p(nw),
                  w_out=self.o_proj.weight.data_ptr(), n_out=self.o_proj.weight.shape[0], skinny_ok={},
-                 w_in=f[0].data_ptr(), bias_ptr=f[1].data_ptr(), skinny_in_ok={},
+                 w_in=f[0].data_ptr(), bias_ptr=f[1].data_ptr(), skinny_in_ok={}, one_call={},
                  keep=(inv_freq, cos_t, sin_t, eta, nw, f, wt))
+        layer = StepLayer(w_in=c["w_in"], bias=c["bias_ptr"], w_out=c["w_out"], inv_freq=c["inv_freq"], eta_logit=c["eta"],
+                          cos_theta=c["cos"], sin_theta=c["sin"], norm_w=c["nw"], embed=f[0].shape[1], npad=c["npad"],
+                          n_heads_out=c["nq"], n_out=c["n_out"], off_k=c["off_k"], off_v=c["off_v"], off_lam=c["off_lam"],
+                          off_gate=c["off_gate"] if c["gated"] else -1)
+        c["layer"], c["layer_ptr"] = layer, C.addressof(layer)
         self.__dict__["_bundle"] = c
         return c
+
+    def _one_call_ok(self, bd, B: int) -> bool:
+        """Whether both projections of a decode step with ``B`` rows run on this library's skinny GEMM with the bundle's
+        weights, so that the step is one native call (``coda_b200_step_layer``)."""
+        ok = bd["one_call"].get(B)
+        if ok is None:
+            W, bias = bd["keep"][5]
+            w = self.o_proj.weight
+            ok = bd["one_call"][B] = bool(
+                W.is_contiguous() and W.data_ptr() % 16 == 0 and bias.data_ptr() % 16 == 0 and bd["npad"] % 8 == 0
+                and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.dtype == torch.bfloat16
+                and lib.coda_b200_skinny_gemm_bias_supported(B, W.shape[1], W.shape[0])
+                and lib.coda_b200_skinny_gemm_supported(B, bd["nq"], w.shape[0]))
+        return ok
 
     def _step_eager_fast(self, x: torch.Tensor, st: CoDAGQALandmarkStatePerf2,
                          residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
@@ -649,6 +668,22 @@ class CoDAGQALandmarkPerf2(nn.Module):
             pc = (kptr, self._ptrs(st), st._exact_v_norm, st._sum_lf_k_norm)
             st.__dict__["_pc"] = pc
         ptrs = pc[1]
+        if self.use_skinny_gemm_kernel and self._one_call_ok(bd, B):
+            xp = x.data_ptr()
+            rp_ = 0 if residual is None else residual.data_ptr()
+            if (x.is_contiguous() and x.shape[2] == self.embed_dim and xp % 16 == 0
+                    and (residual is None or (residual.is_contiguous() and rp_ % 16 == 0 and residual.dtype == x.dtype))):
+                # one workspace (projection rows, then head outputs) and one native call for the step's four launches
+                ws = torch.empty(B * (bd["npad"] + bd["nq"]), device=dev, dtype=x.dtype)
+                y = torch.empty((B, 1, bd["n_out"]), device=dev, dtype=x.dtype)
+                rc = lib.coda_b200_step_layer(bd["layer_ptr"], C.addressof(cfg), C.addressof(ptrs),
+                                              RingPos(st.pos, st.recent_idx, st.recent_filled, None), xp, rp_ or None,
+                                              ws.data_ptr(), y.data_ptr(), self._decode_records(cfg, dev).data_ptr(),
+                                              self._status_word(dev).data_ptr(), _stream(dev))
+                if rc:
+                    check(rc, "coda_b200_step_layer")
+                self.advance_host_scalars(st)
+                return y
         y = None
         if self.use_skinny_gemm_kernel:
             ok = bd["skinny_in_ok"].get(B)

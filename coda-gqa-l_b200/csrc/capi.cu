@@ -123,3 +123,20 @@ extern "C" int coda_b200_step_write_attend(const coda_layer_cfg* cfg, const coda
   if (rc != CODA_OK) return rc;
   return coda_b200_decode_attend_prepared(cfg, st, qrec, norm_w, out, out_bs, status, stream);
 }
+
+extern "C" int coda_b200_step_layer(const coda_step_layer* l, const coda_layer_cfg* cfg, const coda_state_ptrs* st, coda_ring_pos rp,
+                                    const void* x, const void* residual, void* ws, void* y, void* qrec, int32_t* status,
+                                    coda_stream_t stream) {
+  CODA_REQUIRE(l && cfg && ws && cfg->B > 0 && l->npad > 0 && l->npad % 8 == 0 && (uintptr_t)ws % 16 == 0, CODA_ERR_ARG,
+               "step_layer: layer description, workspace or batch size invalid");
+  char* proj = (char*)ws;                                              // (the decode kernels are bf16: two bytes an element)
+  char* heads = proj + (size_t)cfg->B * l->npad * 2;
+  int rc = coda_b200_skinny_gemm_bias(x, cfg->B, l->embed, l->w_in, l->npad, l->bias, nullptr, 0, proj, l->npad, status, stream);
+  if (rc != CODA_OK) return rc;
+  rc = coda_b200_step_write_attend(cfg, st, rp, proj + l->off_k, l->npad, proj + l->off_v, l->npad,
+                                   l->off_gate >= 0 ? proj + l->off_gate : nullptr, l->off_gate >= 0 ? l->npad : 0, l->inv_freq,
+                                   l->eta_logit, proj, l->npad, proj + l->off_lam, l->npad, l->cos_theta, l->sin_theta, qrec,
+                                   l->norm_w, heads, l->n_heads_out, status, stream);
+  if (rc != CODA_OK) return rc;
+  return coda_b200_skinny_gemm(heads, cfg->B, l->n_heads_out, l->w_out, l->n_out, residual, l->n_out, y, l->n_out, status, stream);
+}

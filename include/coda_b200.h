@@ -244,6 +244,23 @@ int coda_b200_skinny_gemm_bias(const void* x, int32_t M, int32_t K, const void* 
                                const void* residual, int64_t res_rs, void* y, int64_t y_rs,
                                int32_t* status, coda_stream_t stream);
 
+/* A whole decode step of one layer in one call: coda_b200_skinny_gemm_bias (fused input projection),
+ * coda_b200_step_write_attend, coda_b200_skinny_gemm (output projection, residual in its epilogue); the same launches
+ * with the same arguments, for callers whose host time per layer counts.  The weights and constants of the layer:
+ * proj rows are [q | k | v | lambda | gate] with `npad` elements, the off_* are byte offsets into a row (off_gate < 0: no
+ * gate). */
+typedef struct coda_step_layer {
+  const void* w_in; const void* bias; const void* w_out;
+  const float* inv_freq; const float* eta_logit; const void* cos_theta; const void* sin_theta; const void* norm_w;
+  int32_t embed, npad, n_heads_out, n_out;
+  int64_t off_k, off_v, off_lam, off_gate;
+} coda_step_layer;
+/* x [B][embed], residual [B][n_out] or null, y [B][n_out]; ws: B * (npad + n_heads_out) elements (projection rows, then head
+ * outputs), 16-byte aligned, npad a multiple of 8. */
+int coda_b200_step_layer(const coda_step_layer* layer, const coda_layer_cfg* cfg, const coda_state_ptrs* st, coda_ring_pos rp,
+                         const void* x, const void* residual, void* ws, void* y, void* qrec, int32_t* status,
+                         coda_stream_t stream);
+
 /* A layer's output projection and the NEXT layer's fused input projection behind one launch:
  *   y_a[M][Na] = x_a[M][Ka] . w_a[Na][Ka]^T (+ residual_a, as coda_b200_skinny_gemm adds it), then
  *   y_b[M][Nb] = y_a . w_b[Nb][Na]^T + bias_b (as coda_b200_skinny_gemm_bias).
