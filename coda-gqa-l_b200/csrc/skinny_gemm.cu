@@ -204,7 +204,10 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
 // owner through distributed shared memory, and the owner adds the four partials (in rank order), bias or residual,
 // and writes.  Launched as a programmatic dependent: the first ring pass of WEIGHT boxes goes out before the wait
 // for the kernel that produces X, and the kernel after this one is let onto the SMs from the start.
-// CW: consumer warps (tiles of up to 16 CW rows); STAGES ring slots of 16 CW x 128 bytes.
+// CW: consumer warps (tiles of up to 16 CW rows); STAGES ring slots of 16 CW x 128 bytes.  MT: 8-token column tiles of the
+// products.  A box of weights costs a warp 4 MT matrix instructions at about 16 cycles each, which at MT = 4 is what
+// paces the ring; calls with at most 8 (16) rows run the instance that leaves the padding out.
+// One row, 4096 -> 6208 and 4096 -> 4096 in a chain of adapters: 14.4 -> 12.4 us a launch, 167 -> 155 us per token for four layers.
 constexpr int S4_CL = 4;
 
 template <int CW, int STAGES>
@@ -224,7 +227,7 @@ struct Skinny4Smem {
   }
 };
 
-template <int CW, int STAGES>
+template <int CW, int STAGES, int MT>
 __global__ void __launch_bounds__((CW + 1) * 32, 1)
 skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, SkinnyParams p, int bn) {
   constexpr int SLOT = Skinny4Smem<CW, STAGES>::SLOT;
@@ -255,9 +258,10 @@ skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   }
   __syncthreads();
 
-  float acc[4][4];
+  constexpr int XBYTES = MT * 8 * 128;                   // X rows asked for per box (its slot holds 32)
+  float acc[MT][4];
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
   const int li = lane >> 3, lr = lane & 7;
 
   if (warp == CW) {
@@ -273,7 +277,7 @@ skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
       for (int i = 0; i < nbox; ++i) {
         if (i % SG_XGROUP == 0) {
           const int g = i / SG_XGROUP, nb = min(SG_XGROUP, nbox - i);
-          tma::mbar_expect_tx(&xbar[g], (uint32_t)nb * SG_XBOX);
+          tma::mbar_expect_tx(&xbar[g], (uint32_t)nb * XBYTES);
           for (int j = 0; j < nb; ++j) sg_tma_load(xs + (i + j) * SG_XBOX, &xmap, &xbar[g], kbase + (i + j) * SG_BK, 0);
         }
         if (i < pre) continue;
@@ -296,7 +300,7 @@ skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) sg_ldsm_x4(a[ks], wb + sg_off(wrow, ks * 2 + (li >> 1)));
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         uint32_t b0[4], b1[4];                           // X^T fragments: k 0-31 and k 32-63 of the box
         sg_ldsm_x4(b0, xb + sg_off(mt * 8 + lr, li));
         sg_ldsm_x4(b1, xb + sg_off(mt * 8 + lr, 4 + li));
@@ -326,7 +330,7 @@ skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     uint32_t base_remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base_remote) : "r"(base_local), "r"(owner));
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) {
+    for (int mt = 0; mt < MT; ++mt) {
       const int tok = mt * 8 + 2 * (lane & 3), nl = lane >> 2;         // C fragment: rows nl, nl + 8 of the group; tokens tok, tok + 1
       const uint32_t a0 = base_remote + (uint32_t)((tok * 16 + nl) * 4);
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a0), "f"(acc[mt][0]) : "memory");
@@ -369,14 +373,14 @@ skinny_gemm4_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
 }
 
 // One instance of the four-way kernel: set-up once per device, clusters that fit at once, launch.
-template <int CW, int STAGES>
+template <int CW, int STAGES, int MT = SG_MAXM / 8>
 struct Skinny4 {
   static int max_clusters(size_t smem) {
     static coda_device_once once;
     static int mc[64];
     const int dev = coda_current_device();
     coda_on_first_use(once, [smem, dev] {
-      cudaFuncSetAttribute(skinny_gemm4_kernel<CW, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+      cudaFuncSetAttribute(skinny_gemm4_kernel<CW, STAGES, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
       cudaLaunchConfig_t q = {};
       q.gridDim = dim3(S4_CL, 64, 1); q.blockDim = dim3((CW + 1) * 32, 1, 1); q.dynamicSmemBytes = smem;
       cudaLaunchAttribute qa[1];
@@ -384,14 +388,21 @@ struct Skinny4 {
       qa[0].val.clusterDim.x = S4_CL; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
       q.attrs = qa; q.numAttrs = 1;
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, skinny_gemm4_kernel<CW, STAGES>, &q) != cudaSuccess) { n = 0; cudaGetLastError(); }
+      if (cudaOccupancyMaxActiveClusters(&n, skinny_gemm4_kernel<CW, STAGES, MT>, &q) != cudaSuccess) { n = 0; cudaGetLastError(); }
       if (dev >= 0 && dev < 64) mc[dev] = n;
     });
     return (dev >= 0 && dev < 64) ? mc[dev] : 0;
   }
-  static int launch(const CUtensorMap& xm, const void* w, const SkinnyParams& p, int bn, size_t smem, cudaStream_t stream) {
-    CUtensorMap wm;
-    CODA_REQUIRE(tmaps::plane_map(&wm, w, 1, p.N, p.K, bn), CODA_ERR_LAUNCH, "skinny_gemm: cuTensorMapEncodeTiled failed");
+  static int launch(const void* x, const void* w, const SkinnyParams& p, int bn, size_t smem, cudaStream_t stream) {
+    CUtensorMap xm, wm;
+    CODA_REQUIRE(tmaps::plane_map(&xm, x, 1, p.M, p.K, MT * 8) && tmaps::plane_map(&wm, w, 1, p.N, p.K, bn), CODA_ERR_LAUNCH,
+                 "skinny_gemm: cuTensorMapEncodeTiled failed");
+    if (MT != SG_MAXM / 8) {                             // (the plan has set the largest instance up)
+      static coda_device_once once;
+      coda_on_first_use(once, [] {
+        cudaFuncSetAttribute(skinny_gemm4_kernel<CW, STAGES, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+      });
+    }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(S4_CL, (p.N + bn - 1) / bn, 1);
     lc.blockDim = dim3((CW + 1) * 32, 1, 1);
@@ -403,11 +414,20 @@ struct Skinny4 {
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&lc, skinny_gemm4_kernel<CW, STAGES>, xm, wm, p, bn);
+    cudaError_t e = cudaLaunchKernelEx(&lc, skinny_gemm4_kernel<CW, STAGES, MT>, xm, wm, p, bn);
     if (e != cudaSuccess) { coda_set_error("skinny_gemm (four-way): %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
     return CODA_OK;
   }
 };
+
+// ... and the instance for the number of rows
+template <int CW, int STAGES>
+int skinny4_launch(const void* x, const void* w, const SkinnyParams& p, int bn, cudaStream_t stream) {
+  const size_t smem = (size_t)Skinny4Smem<CW, STAGES>(p.K / S4_CL).total + 1024;
+  if (p.M <= 8) return Skinny4<CW, STAGES, 1>::launch(x, w, p, bn, smem, stream);
+  if (p.M <= 16) return Skinny4<CW, STAGES, 2>::launch(x, w, p, bn, smem, stream);
+  return Skinny4<CW, STAGES>::launch(x, w, p, bn, smem, stream);
+}
 
 // ---- two dependent products behind one launch -------------------------------------------------------------------
 // A decode step's output projection (with the residual) is followed by the next layer's input projection, whose X is
@@ -679,8 +699,6 @@ extern "C" int coda_b200_skinny_gemm_bias(const void* x, int32_t M, int32_t K, c
   CODA_REQUIRE(!residual || ((uintptr_t)residual % 16 == 0 && res_rs % 8 == 0 && res_rs >= N), CODA_ERR_ARG,
                "skinny_gemm: misaligned residual");
   CODA_REQUIRE(!bias || (uintptr_t)bias % 16 == 0, CODA_ERR_ARG, "skinny_gemm: misaligned bias");
-  CUtensorMap xm, wm;
-  CODA_REQUIRE(tmaps::plane_map(&xm, x, 1, M, K, SG_MAXM), CODA_ERR_LAUNCH, "skinny_gemm: cuTensorMapEncodeTiled failed");
   SkinnyParams p;
   p.M = M; p.N = N; p.K = K; p.res = (const bf16*)residual; p.res_rs = res_rs; p.bias = (const bf16*)bias;
   p.y = (bf16*)y; p.y_rs = y_rs; p.status = status;
@@ -688,11 +706,13 @@ extern "C" int coda_b200_skinny_gemm_bias(const void* x, int32_t M, int32_t K, c
   int cw = 0;
   const int bn = skinny4_plan(K, N, &cw);
   if (bn != 0) {
-    if (cw == 8) return Skinny4<8, 8>::launch(xm, w, p, bn, (size_t)Skinny4Smem<8, 8>(K / 4).total + 1024, (cudaStream_t)stream);
-    return Skinny4<12, 6>::launch(xm, w, p, bn, (size_t)Skinny4Smem<12, 6>(K / 4).total + 1024, (cudaStream_t)stream);
+    if (cw == 8) return skinny4_launch<8, 8>(x, w, p, bn, (cudaStream_t)stream);
+    return skinny4_launch<12, 6>(x, w, p, bn, (cudaStream_t)stream);
   }
   CODA_REQUIRE(!bias, CODA_ERR_LIMIT, "skinny_gemm: the bias epilogue needs the four-way kernel, which does not cover %d x %d -> %d here", M, K, N);
-  CODA_REQUIRE(tmaps::plane_map(&wm, w, 1, N, K, SG_BN), CODA_ERR_LAUNCH, "skinny_gemm: cuTensorMapEncodeTiled failed");
+  CUtensorMap xm, wm;
+  CODA_REQUIRE(tmaps::plane_map(&xm, x, 1, M, K, SG_MAXM) && tmaps::plane_map(&wm, w, 1, N, K, SG_BN), CODA_ERR_LAUNCH,
+               "skinny_gemm: cuTensorMapEncodeTiled failed");
   const size_t smem = (size_t)SkinnySmem(K / 2).total + 1024;
   static coda_device_once once;
   coda_on_first_use(once, [] {

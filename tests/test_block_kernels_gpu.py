@@ -139,3 +139,27 @@ def test_batched_routing_head_dim_64(kw, B):
         assert torch.equal(a.k_buf[:, :, W:], b.k_buf[:, :, W:]) and torch.equal(a.v_buf[:, :, W:], b.v_buf[:, :, W:])
         assert torch.equal(a._exact_v_norm, b._exact_v_norm) and torch.equal(a._sum_lf_k_norm, b._sum_lf_k_norm)
     assert all(layer.device_status() == 0 for layer in layers)
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 24, 25, 32])
+@pytest.mark.parametrize("K,N,bias,res", [(512, 832, True, False), (4096, 4096, False, True), (1024, 6208, True, True)])
+def test_skinny_gemm_row_instances(M, K, N, bias, res):
+    """Every number of 8-row tiles of the four-way kernel against the product in 64 bits: fp32 sums, one rounding of the product
+    and one of the sum with the residual (2^-8 of a value together, in the norm well below)."""
+    from coda_gqa_l_b200 import _lib as b
+    g = torch.Generator("cuda").manual_seed(M + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, w = rnd(M, K), rnd(N, K)
+    bv, rv = (rnd(N) if bias else None), (rnd(M, N) if res else None)
+    y = torch.full((M + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    b.check(b.lib.coda_b200_skinny_gemm_bias(x.data_ptr(), M, K, w.data_ptr(), N, p(bv), p(rv), N, y.data_ptr(), N, status.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream), "skinny")
+    want = x.double() @ w.double().t()
+    if bias:
+        want = want + bv.double()
+    if res:
+        want = want + rv.double()
+    assert status.item() == 0 and torch.isnan(y[M]).all()
+    assert rel_err(y[:M], want) < 4e-3
