@@ -35,6 +35,7 @@ namespace {
 
 constexpr int DA_TILE = 64;          // slots per stage
 constexpr int DA_MAX_STAGES = 8;
+constexpr int DA_BUDGET = 226 * 1024;   // shared memory of an SM that the CTAs of this kernel share
 constexpr int DA_CWARPS = 8;         // consumer warps (two groups of four)
 constexpr int DA_AWARPS = 4;         // auxiliary warps (query preparation, merge + epilogue)
 constexpr int DA_THREADS = (DA_CWARPS + DA_AWARPS + 1) * 32;   // 8 consumer, 4 auxiliary, 1 producer warp
@@ -189,10 +190,10 @@ __global__ void __launch_bounds__(128) decode_prep_kernel(DecodeParams p, const 
 // CTAs per SM: a plane is a chain (record, tiles, hand-over, merge) that the three roles overlap with the next plane's,
 // but where a plane holds few bytes (head_dim 64) the roles' own chains are longer than its tiles take to arrive, so
 // two CTAs share an SM there, each with half of the ring: 28.1 -> 23.4 us for 512 states x 3 heads of 192 slots.
-constexpr int da_ctas(int dh, int nq) { return dh == 64 && nq == 1 ? 2 : 1; }   // (16 query rows do not fit half the registers)
-
-template <int DH, int NQ, bool APPEND>
-__global__ void __launch_bounds__(DA_THREADS, da_ctas(DH, NQ))
+// (16 query rows do not fit half the registers, and calls with no more planes than SMs keep one CTA per SM, all its
+// registers and the whole ring.)
+template <int DH, int NQ, bool APPEND, int CTAS>
+__global__ void __launch_bounds__(DA_THREADS, CTAS)
 decode_attend_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, DecodeParams p) {
   constexpr int KSTEPS = DH / 16;            // k-steps of Q.K^T
   constexpr int MT_O = DH / 16;              // m-tiles of the (transposed) output
@@ -713,29 +714,27 @@ decode_attend_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
   }  // plane loop
 }
 
-template <int DH, int NQ, bool APPEND>
-int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, DecodeParams p, cudaStream_t s) {
-  constexpr int BUDGET = 226 * 1024;
+template <int DH, int NQ, bool APPEND, int CTAS>
+int launch_decode_ctas(const CUtensorMap& km, const CUtensorMap& vm, DecodeParams p, cudaStream_t s) {
+  constexpr int BUDGET = DA_BUDGET / CTAS;
   // as many ring stages as fit beside the fixed buffers (at least 2, at most DA_MAX_STAGES)
   const int fixed = DecodeSmem<DH>(0, p.G, p.Lbuf).total + 1024;
-  static coda_device_once once;
-  const int num_sms = coda_on_first_use(once, [] {
-    cudaFuncSetAttribute(decode_attend_kernel<DH, NQ, APPEND>, cudaFuncAttributeMaxDynamicSharedMemorySize, BUDGET);
-  });
-  const int nplanes = p.B * p.Hkv;
-  // (no more planes than SMs, or a ring that half an SM cannot hold: one CTA per SM takes the whole budget)
-  const int ctas = nplanes > num_sms && (BUDGET / da_ctas(DH, NQ) - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES) >= 2 ? da_ctas(DH, NQ) : 1;
-  int stages = (BUDGET / ctas - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES);
+  int stages = (BUDGET - fixed) / (2 * DecodeSmem<DH>::TILE_BYTES);
   if (stages > DA_MAX_STAGES) stages = DA_MAX_STAGES;
   stages &= ~1;                                      // even: each ring stage belongs to one consumer group (see the kernel)
   CODA_REQUIRE(stages >= 2, CODA_ERR_LIMIT, "decode_attend: %d slots leave no room for the tile ring in shared memory", p.Lbuf);
   p.stages = stages;
   const size_t smem = (size_t)DecodeSmem<DH>(stages, p.G, p.Lbuf).total + 1024;
+  static coda_device_once once;
+  const int num_sms = coda_on_first_use(once, [] {
+    cudaFuncSetAttribute(decode_attend_kernel<DH, NQ, APPEND, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DA_BUDGET);
+  });
+  const int nplanes = p.B * p.Hkv;
   // Programmatic dependent launch: the CTAs may start (shared-memory carve-up, barrier initialisation) while the
   // kernel before this one on the stream is still finishing; they wait for it (griddepcontrol.wait) before the
   // first global access.
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(nplanes < ctas * num_sms ? nplanes : ctas * num_sms, 1, 1);
+  lc.gridDim = dim3(nplanes < CTAS * num_sms ? nplanes : CTAS * num_sms, 1, 1);
   lc.blockDim = dim3(DA_THREADS, 1, 1);
   lc.dynamicSmemBytes = smem;
   lc.stream = s;
@@ -743,9 +742,20 @@ int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, DecodeParams p, 
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at; lc.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&lc, decode_attend_kernel<DH, NQ, APPEND>, km, vm, p);
+  cudaError_t e = cudaLaunchKernelEx(&lc, decode_attend_kernel<DH, NQ, APPEND, CTAS>, km, vm, p);
   if (e != cudaSuccess) { coda_set_error("decode_attend: %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
   return CODA_OK;
+}
+
+template <int DH, int NQ, bool APPEND>
+int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, const DecodeParams& p, cudaStream_t s) {
+  if constexpr (DH == 64 && NQ == 1) {
+    static coda_device_once once;
+    const int num_sms = coda_on_first_use(once, [] {});
+    const bool fits = (DA_BUDGET / 2 - DecodeSmem<DH>(0, p.G, p.Lbuf).total - 1024) / (2 * DecodeSmem<DH>::TILE_BYTES) >= 2;
+    if (p.B * p.Hkv > num_sms && fits) return launch_decode_ctas<DH, NQ, APPEND, 2>(km, vm, p, s);
+  }
+  return launch_decode_ctas<DH, NQ, APPEND, 1>(km, vm, p, s);
 }
 
 int check_common(const coda_layer_cfg* cfg, const coda_state_ptrs* st, const void* qrec, const void* norm_w, const void* out) {
