@@ -965,7 +965,8 @@ __global__ void __launch_bounds__(256) step_write_cluster_kernel(StepParams p) {
 // device array.  The routing of one layer is a latency chain that keeps an SM's resources while it waits; all
 // layers' chains side by side fill the machine and are bounded by memory bandwidth instead.
 // The chain is as long with 128 threads as with 256 and a CTA needs no more of them at Dh 64, so there twice as many
-// chains share an SM: 122 -> 86 us for 8 layers x 512 states x 3 heads.
+// chains share an SM: 122 -> 86 us for 8 layers x 512 states x 3 heads.  As long as every chain is resident at once with 256
+// threads (five CTAs per SM) the wider CTA is the faster one (80 chains: 29.1 against 30.2 us per one-layer step).
 template <typename T, int DH, bool STAGE, int NCTA, int NT>
 __global__ void __launch_bounds__(NT, NCTA) step_route_batched_kernel(const StepParams* __restrict__ layers) {
   __shared__ StepParams sp;
@@ -1184,7 +1185,10 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
   const int MM = cfg->Me + cfg->Ms;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(cfg->Hkv, cfg->B, n_layers);
-  lc.blockDim = dim3(cfg->Dh == 128 ? 256 : 128, 1, 1);
+  static coda_device_once once;
+  const int num_sms = coda_on_first_use(once, [] {});
+  const bool narrow = cfg->Dh == 64 && (long long)cfg->Hkv * cfg->B * n_layers > 5LL * num_sms;      // 128-thread CTAs, see the kernel
+  lc.blockDim = dim3(narrow ? 128 : 256, 1, 1);
   lc.dynamicSmemBytes = sizeof(float) * ((size_t)cfg->Hkv * MM + MM) + 8 + 8 * (size_t)cfg->Me + (size_t)(cfg->W + MM) + 16;
   lc.stream = (cudaStream_t)stream;
   cudaLaunchAttribute at[1];
@@ -1201,10 +1205,12 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
     lc.dynamicSmemBytes += 16 + stage_bytes;
     // five CTAs per SM measured best at the 7B shape (4: 122 us, 5: 111 us, 6: 114 us for 32 layers x 32 states)
     e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, true, 5, 256>, plan)
-                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 10, 128>, plan);
+        : narrow         ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 10, 128>, plan)
+                         : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 5, 256>, plan);
   } else {
     e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, false, 4, 256>, plan)
-                       : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 8, 128>, plan);
+        : narrow         ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 8, 128>, plan)
+                         : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 4, 256>, plan);
   }
   if (e != cudaSuccess) { coda_set_error("step_route_batched: %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
   return CODA_OK;
