@@ -254,10 +254,15 @@ class CoDAGQALandmarkPerf2(nn.Module):
             raise ValueError("mem_init must be 'zeros' or 'random_normal'")
         st.active_exact = self.Me_min if Me > 0 else 0
         st.active_summary = self.Ms_min if Ms > 0 else 0
-        if Me > 0:
-            st._exact_v_norm.copy_(F.normalize(st.v_buf[:, :, W:W + Me, :], dim=-1, eps=1e-6))
-        if Ms > 0:
-            st._sum_lf_k_norm.copy_(F.normalize(st.k_buf[:, :, W + Me:, self.lf_start:], dim=-1, eps=1e-6))
+        if st.k_buf.is_cuda and st.k_buf.device.index == torch.cuda.current_device() and 0 < B <= 65535:
+            # both routing caches in one launch
+            cfg = LayerCfg(B=B, H=self.num_heads, Hkv=self.num_kv_heads, Dh=self.head_dim, W=W, Me=Me, Ms=Ms, dtype=_DT[dtype])
+            check(lib.coda_b200_bank_norms(C.byref(cfg), C.byref(self._ptrs(st)), _stream(st.k_buf.device)), "coda_b200_bank_norms")
+        else:
+            if Me > 0:
+                st._exact_v_norm.copy_(F.normalize(st.v_buf[:, :, W:W + Me, :], dim=-1, eps=1e-6))
+            if Ms > 0:
+                st._sum_lf_k_norm.copy_(F.normalize(st.k_buf[:, :, W + Me:, self.lf_start:], dim=-1, eps=1e-6))
         if self.collect_metrics:
             st.metrics = new_metrics(st.active_exact, st.active_summary)
         return st

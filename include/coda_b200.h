@@ -244,6 +244,11 @@ int coda_b200_skinny_gemm_bias(const void* x, int32_t M, int32_t K, const void* 
                                const void* residual, int64_t res_rs, void* y, int64_t y_rs,
                                int32_t* status, coda_stream_t stream);
 
+/* Routing caches of a fresh state from its bank slots: exact_v_norm = unit vectors of the exact bank's values, sum_lf_k_norm
+ * = unit vectors of the phase-safe half of the summary bank's keys (src/coda_gqa_l/attention.py:300-317).  Of `cfg` only
+ * the sizes and the dtype are read. */
+int coda_b200_bank_norms(const coda_layer_cfg* cfg, const coda_state_ptrs* st, coda_stream_t stream);
+
 /* A whole decode step of one layer in one call: coda_b200_skinny_gemm_bias (fused input projection),
  * coda_b200_step_write_attend, coda_b200_skinny_gemm (output projection, residual in its epilogue); the same launches
  * with the same arguments, for callers whose host time per layer counts.  The weights and constants of the layer:

@@ -163,3 +163,22 @@ def test_skinny_gemm_row_instances(M, K, N, bias, res):
         want = want + rv.double()
     assert status.item() == 0 and torch.isnan(y[M]).all()
     assert rel_err(y[:M], want) < 4e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,Hkv,Dh,Me,Ms", [(4, 2, 64, 7, 5), (2, 1, 20, 1, 0), (8, 8, 128, 0, 33), (2, 2, 64, 0, 0)])
+def test_routing_caches_of_a_fresh_state(dtype, H, Hkv, Dh, Me, Ms):
+    """The one-launch unit vectors against torch's normalisation of the same slots, zeros for zero rows.  The norm's 32-bit sum
+    runs in another order: at most 7 roundings each way, halved by the root, and one of the quotient, below 2^-21; in bf16 a
+    norm or a quotient that falls on the other side moves by one step, at most 2^-7."""
+    from torch.nn import functional as F
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    mod = CoDAGQALandmarkPerf2(embed_dim=H * Dh, num_heads=H, num_kv_heads=Hkv, window=6, num_landmarks_exact=Me,
+                               num_landmarks_summary=Ms).eval().to(dtype).cuda()
+    ulp = 2.0 ** -21 if dtype == torch.float32 else 2.0 ** -7
+    for init in ("random_normal", "zeros"):
+        st = mod.init_state(batch_size=3, device="cuda", dtype=dtype, mem_init=init)
+        for got, src in ((st._exact_v_norm, st.v_buf[:, :, 6:6 + Me]), (st._sum_lf_k_norm, st.k_buf[:, :, 6 + Me:, Dh // 2:])):
+            if got is not None:
+                assert torch.allclose(got.double(), F.normalize(src, dim=-1, eps=1e-6).double(), rtol=ulp, atol=0)
+
