@@ -7,15 +7,17 @@
 //     S = Q . K^T          tcgen05.mma  M=128 N=64 K=Dh    A, B from shared memory, S in TMEM
 //     P = exp2(S - m)      softmax warps: tcgen05.ld, lazy-rescaled online softmax, bf16 P written back over S
 //     O += P . V           tcgen05.mma  M=128 N=Dh K=64    A = P straight from TMEM, B = V from shared memory
-// Warp roles: warps 0-3 = softmax / correction / epilogue (one thread per row), warp 4 = TMA producer (128-byte
-// swizzle, K and V on rings of their own), warp 5 = MMA issuer and TMEM owner.
-// What bounds it: the softmax warps' issue slots and special-function work.  Everything else is arranged so that they
-// do not wait.  S is double-buffered (S0, S1: 128 TMEM columns; with O at most 256), so Q.K^T of the next tile is
-// complete before the softmax of the present one ends, and half the tensor memory per CTA lets two CTAs share an SM:
-// one CTA's start-up and epilogue (a third of a CTA's life) run under the other's tiles.
-// Measured per block (two streams of 128 rows in one CTA per SM, 128-key tiles, before): 64 states x 8 heads x 256 queries
-// over 384 slots, Dh 64: 109 -> 94 us; 512 x 9 x 128 over 192, Dh 64: 352 -> 258 us; 32 x 32 x 128 over 384, Dh 128:
-// 115 -> 104 us; 8 x 64 x 256 over 768, Dh 128: 179 -> 165 us; 1 x 32 x 1000 over an empty state, Dh 128: 59 -> 42 us.
+// Warp roles: warps 0-7 = softmax / correction / epilogue (two warps per 32 rows, each with 32 of a tile's 64 keys),
+// warp 8 = TMA producer (128-byte swizzle, K and V on rings of their own), warp 9 = MMA issuer and TMEM owner.
+// What bounds it: the chain of a tile (S from TMEM, maximum, exponentials, P back), 1.6 K cycles a CTA-tile against 0.44 K
+// for the exponentials' instructions alone; no pipe is more than half busy.  So everything is arranged to keep that
+// chain short and several of them in flight.  S is double-buffered (S0, S1: 128 TMEM columns; with O at most 256), so
+// Q.K^T of the next tile runs under the softmax of the present one, and half the tensor memory per CTA lets two CTAs share
+// an SM: one CTA's start-up and epilogue (some 7 K cycles) run under the other's tiles.  64-key tiles are what fits twice;
+// 64 queries x 2 streams fill the 128 rows of an MMA.
+// Measured per block, against two streams of 128 rows in one CTA per SM with 128-key tiles: 64 states x 8 heads x 256
+// queries over 384 slots, Dh 64: 109 -> 88 us; 512 x 9 x 128 over 192, Dh 64: 352 -> 241 us; 32 x 32 x 128 over 384, Dh
+// 128: 115 -> 90 us; 8 x 64 x 256 over 768, Dh 128: 179 -> 131 us.
 // All mbarrier waits are bounded (status word, no hang, TMEM is freed).
 #include "coda_common.cuh"
 #include "tma_utils.cuh"

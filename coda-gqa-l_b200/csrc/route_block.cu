@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
 // layer left three threads in four idle and the chip waiting on CTA launches.
 // Per block: 40 -> 12.5 us (64 states, 2 x 64 elements a row), 233 -> 91 us (512 states, 3 x 64), 31 -> 22 us (32 states, 8 x 128).
 template <typename T, int WPS, bool PACKED>
-__global__ void __launch_bounds__(WPS == 8 ? 256 : 128, WPS == 8 ? 3 : 6) route_apply_kernel(RouteParams p, int nslots) {
+__global__ void __launch_bounds__(WPS == 8 ? 256 : 128, WPS == 8 ? 4 : WPS == 1 ? 8 : 6) route_apply_kernel(RouteParams p, int nslots) {
   extern __shared__ float stash_all[];                               // [groups of the CTA][Hkv*Dh] new rows for re-normalising
   const coda_layer_cfg& c = p.c;
   constexpr int GT = 32 * WPS, GROUPS = (WPS == 8 ? 256 : 128) / GT; // threads of a slot's group, groups per CTA
