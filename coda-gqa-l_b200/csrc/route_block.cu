@@ -456,19 +456,18 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
   long long* last = (long long*)p.st.mem_last_exact + (long long)b * Me;
   Plan pl = plan_of(p, b);
   const int Ae = c.active_exact;
-  grid_chain();
+  // All but the scores was there before the scoring kernel passed its own wait (it lets this one come only then) and is not
+  // written by it: candidates, gates, flags and stamps are read (through L2), and the victims ranked, while it still runs.
   for (int t = tid; t < tmax; t += NT) {
-    const int e = p.cand[(long long)b * p.cand_bs + t];
+    const int e = __ldcg(p.cand + (long long)b * p.cand_bs + t);
     c_e[t] = e;
-    c_g[t] = p.gates[(long long)b * p.gates_bs + p.gate_ev0 + e];
+    c_g[t] = __ldcg(p.gates + (long long)b * p.gates_bs + p.gate_ev0 + e);
   }
-  for (int t = tid; t < te; t += NT) { x_best[t] = p.ex_best[(long long)b * c.Te + t]; x_bi[t] = p.ex_bi[(long long)b * c.Te + t]; }
-  for (int t = tid; t < ts; t += NT) s_idx[t] = p.su_idx[(long long)b * c.Ts + t];
-  for (int m = tid; m < Ms; m += NT) s_used[Me + m] = al[W + Me + m];
+  for (int m = tid; m < Ms; m += NT) s_used[Me + m] = __ldcg(al + W + Me + m);
   int used_here = 0;
   for (int m = tid; m < Me; m += NT) {
-    const bool used = al[W + m] != 0;
-    const long long stamp = last[m];
+    const bool used = __ldcg(al + W + m) != 0;
+    const long long stamp = __ldcg(last + m);
     s_used[m] = used;
     s_last[m] = stamp;
     lruq[m].v = (used && m < Ae) ? stamp : -(1LL << 62);
@@ -476,15 +475,19 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
     n_first[m] = 0x7fffffff; n_e[m] = -1;
     used_here |= used ? 1 : 0;
   }
+  const bool any_used = __syncthreads_or(used_here) != 0;
+  const int n_lru = te < Ae ? te : Ae;
+  if (tid < 32 && te > 0) topk_order::topk_queue_warp<long long, false>(lruq, Me, n_lru, true, qscr);   // victims = lruq[0..n_lru).i
+  grid_chain();
+  for (int t = tid; t < te; t += NT) { x_best[t] = p.ex_best[(long long)b * c.Te + t]; x_bi[t] = p.ex_bi[(long long)b * c.Te + t]; }
+  for (int t = tid; t < ts; t += NT) s_idx[t] = p.su_idx[(long long)b * c.Ts + t];
   // routing-event record of this call (optional): cleared here, filled by the deciding warps below
   int32_t* evw = p.st.events != nullptr ? p.st.events + (long long)b * CODA_EVENT_WORDS : nullptr;
   if (evw != nullptr && tid < CODA_EVENT_WORDS) evw[tid] = 0;
-  const bool any_used = __syncthreads_or(used_here) != 0;
+  __syncthreads();
   if (tid < 32) {
     if (te > 0) {
       // ---- exact bank (memory_banks.py:635-697) ----
-      const int n_lru = te < Ae ? te : Ae;
-      topk_order::topk_queue_warp<long long, false>(lruq, Me, n_lru, true, qscr);   // victims = lruq[0..n_lru).i
       const float tn = El<T>::rnd(c.tau_novel), tm = El<T>::rnd(c.tau_match);
       int ranked = 0, n_gated = 0, n_hit = 0, n_ins = 0, n_ow = 0, n_frus = 0;
       for (int t0 = 0; t0 < te; t0 += 32) {
