@@ -15,6 +15,7 @@
 // three rows in four of the larger tile would be padding.
 #include "coda_common.cuh"
 #include "attend_f32.h"
+#include <type_traits>
 
 namespace {
 
@@ -170,26 +171,34 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
     }
     cp_wait<1>();                              // this tile's V (the next K is the younger group)
     __syncwarp();
+    // A key behind a row's causal limit is left out, not multiplied by its zero weight: a token whose values are
+    // infinite or not a number must not reach the outputs of the tokens before it.  Only the tiles that hold the
+    // diagonal ask.
+    auto accumulate = [&](auto diagonal) {
 #pragma unroll 4
-    for (int kk = 0; kk < AF_TK; ++kk) {
-      float w[TM];
-      if constexpr (TM == 4) {
-        const float4 pv = *reinterpret_cast<const float4*>(Ps + kk * PS + rg * 4);
-        w[0] = pv.x; w[1] = pv.y; w[2] = pv.z; w[3] = pv.w;
-      } else {
+      for (int kk = 0; kk < AF_TK; ++kk) {
+        float w[TM];
+        if constexpr (TM == 4) {
+          const float4 pv = *reinterpret_cast<const float4*>(Ps + kk * PS + rg * 4);
+          w[0] = pv.x; w[1] = pv.y; w[2] = pv.z; w[3] = pv.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < TM; ++i) w[i] = Ps[kk * PS + rg * TM + i];
-      }
+          for (int i = 0; i < TM; ++i) w[i] = Ps[kk * PS + rg * TM + i];
+        }
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float4 vv = *reinterpret_cast<const float4*>(Vs + kk * DH + (kg + 8 * c) * 4);
+        for (int c = 0; c < NC; ++c) {
+          const float4 vv = *reinterpret_cast<const float4*>(Vs + kk * DH + (kg + 8 * c) * 4);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          acc[i][4 * c] = fmaf(w[i], vv.x, acc[i][4 * c]); acc[i][4 * c + 1] = fmaf(w[i], vv.y, acc[i][4 * c + 1]);
-          acc[i][4 * c + 2] = fmaf(w[i], vv.z, acc[i][4 * c + 2]); acc[i][4 * c + 3] = fmaf(w[i], vv.w, acc[i][4 * c + 3]);
+          for (int i = 0; i < TM; ++i) {
+            if (diagonal.value && t * AF_TK + kk > p.Lbuf + q0 + (rg * TM + i) % BQ) continue;
+            acc[i][4 * c] = fmaf(w[i], vv.x, acc[i][4 * c]); acc[i][4 * c + 1] = fmaf(w[i], vv.y, acc[i][4 * c + 1]);
+            acc[i][4 * c + 2] = fmaf(w[i], vv.z, acc[i][4 * c + 2]); acc[i][4 * c + 3] = fmaf(w[i], vv.w, acc[i][4 * c + 3]);
+          }
         }
       }
-    }
+    };
+    if ((t + 1) * AF_TK > p.Lbuf + q0 + 1 && has_blk) accumulate(std::true_type());
+    else accumulate(std::false_type());
     __syncwarp();
     if (tn < ntiles) load(Vs, DH, vbase, vblk, p.vb_rs, tn); else cp_commit();
     t = tn; bits = nbits;

@@ -75,6 +75,34 @@ def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
     assert rel_err(out, y.transpose(1, 2).reshape(B, Lq, H * Dh)) < 5e-6
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("Dh", [32, 64, 128])
+def test_single_precision_attention_keeps_later_tokens_out(Dh, bad):
+    """A token whose values are infinite or not a number leaves the outputs of the block's earlier tokens as they are, bit for
+    bit, wherever it stands in the query and key tiles."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    mod = CoDAGQALandmarkPerf2(embed_dim=2 * Dh, num_heads=2, num_kv_heads=1, window=40, num_landmarks_exact=0,
+                               num_landmarks_summary=0).eval().cuda()
+    st = mod.init_state(batch_size=1, device="cuda", dtype=torch.float32)
+    g = torch.Generator("cuda").manual_seed(Dh)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    st.k_buf.copy_(rnd(*st.k_buf.shape))
+    st.v_buf.copy_(rnd(*st.v_buf.shape))
+    st.allowed.fill_(True)
+    cfg = mod._cfg(1, torch.float32, st)
+    for Lq in (2, 3, 9, 40):
+        q, qn, lam = rnd(1, Lq, 2 * Dh), rnd(1, Lq, 2 * Dh), torch.rand(1, Lq, 2, generator=g, device="cuda")
+        k, v = rnd(1, Lq, Dh), rnd(1, Lq, Dh)
+        want, out = torch.empty_like(q), torch.empty_like(q)
+        mod._attend(cfg, st, Lq, q, qn, lam, k, v, want)
+        for t in range(1, Lq):
+            spoiled = v.clone()
+            spoiled[0, t] = bad
+            mod._attend(cfg, st, Lq, q, qn, lam, k, spoiled, out)
+            assert torch.equal(out[:, :t], want[:, :t]), (Lq, t)
+            assert not torch.isfinite(out[:, t:]).any()
+
+
 @pytest.mark.parametrize("kw,Te,Ts,block,B", [
     # one warp per slot: more candidates than a warp has lanes, more than 16 LRU victims, slot counts that are not
     # multiples of 32, one and several tiles of scores
