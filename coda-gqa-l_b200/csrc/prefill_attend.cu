@@ -16,8 +16,8 @@
 // an SM: one CTA's start-up and epilogue (some 7 K cycles) run under the other's tiles.  64-key tiles are what fits twice;
 // 64 queries x 2 streams fill the 128 rows of an MMA.
 // Measured per block, against two streams of 128 rows in one CTA per SM with 128-key tiles: 64 states x 8 heads x 256
-// queries over 384 slots, Dh 64: 109 -> 88 us; 512 x 9 x 128 over 192, Dh 64: 352 -> 241 us; 32 x 32 x 128 over 384, Dh
-// 128: 115 -> 90 us; 8 x 64 x 256 over 768, Dh 128: 179 -> 131 us.
+// queries over 384 slots, Dh 64: 109 -> 91 us; 512 x 9 x 128 over 192, Dh 64: 352 -> 254 us; 32 x 32 x 128 over 384, Dh
+// 128: 115 -> 95 us; 8 x 64 x 256 over 768, Dh 128: 179 -> 137 us.
 // All mbarrier waits are bounded (status word, no hang, TMEM is freed).
 #include "coda_common.cuh"
 #include "tma_utils.cuh"
@@ -357,30 +357,26 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint32_t o_col = lane_addr + TM_O;
 
-    float mb = -INFINITY;                                 // exponent base (lags the true max by < GAP), the same in both halves
-    float l = 0.f;                                        // sum over this warp's keys
-    for (int it = 0; it < NT; ++it) {
-      const uint32_t s_col = lane_addr + (uint32_t)(it & 1) * PF_BN;
-      // Visibility of this warp's 32 keys.  cls: 2 = all visible, 0 = none, 1 = mixed; the class is the same for
-      // every lane of a warp: prefix slots carry one mask per state, and in a block tile the 32 rows of a warp
-      // meet the causal diagonal inside one group only.
-      uint32_t vis; int cls;
+    // Visibility of this warp's 32 keys of a tile.  The class (2 = all visible, 0 = none, 1 = mixed) is the same for
+    // every lane of a warp: prefix slots carry one mask per state, and in a block tile the 32 rows of a warp
+    // meet the causal diagonal inside one group only.
+    auto visible = [&](int it, uint32_t& vis) {
       if (it < NV) {
         vis = sMask[2 * it + hf];
-        cls = vis == 0xffffffffu ? 2 : (vis == 0u ? 0 : 1);
-      } else {
-        const int c0 = (it - NV) * PF_BN + 32 * hf;
-        const int nvis = grow - c0 + 1;                   // key c0+i visible iff c0+i <= grow
-        const int gd = (r0 + (quarter & 1) * 32 - c0) >> 5;       // 0: this group holds the warp's diagonal
-        vis = nvis >= 32 ? 0xffffffffu : (nvis <= 0 ? 0u : ((1u << nvis) - 1u));
-        cls = gd > 0 ? 2 : (gd == 0 ? 1 : 0);
+        return vis == 0xffffffffu ? 2 : (vis == 0u ? 0 : 1);
       }
+      const int c0 = (it - NV) * PF_BN + 32 * hf;
+      const int nvis = grow - c0 + 1;                     // key c0+i visible iff c0+i <= grow
+      const int gd = (r0 + (quarter & 1) * 32 - c0) >> 5; // 0: this group holds the warp's diagonal
+      vis = nvis >= 32 ? 0xffffffffu : (nvis <= 0 ? 0u : ((1u << nvis) - 1u));
+      return gd > 0 ? 2 : (gd == 0 ? 1 : 0);
+    };
+    // This warp's part of S of a tile, and the row maximum over its visible keys (the others become -inf)
+    auto load_s = [&](int it, uint32_t vis, int cls, uint32_t (&v)[32]) {
       tma::mbar_wait(&s_full[it & 1], (it >> 1) & 1, p.status, 16, abortw);
       tc_fence_after();
-      uint32_t v[32];
-      tc_ld32(s_col + hf * 32, v);
+      tc_ld32(lane_addr + (uint32_t)(it & 1) * PF_BN + hf * 32, v);
       tc_wait_ld();
-      // row maximum over the visible keys
       float m0 = -INFINITY, m1 = -INFINITY;
       if (cls == 2) {
 #pragma unroll
@@ -395,7 +391,30 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
           m0 = fmaxf(m0, __uint_as_float(v[i]));
         }
       }
-      float mx = fmaxf(m0, m1) * p.scale_log2;            // scale > 0: max commutes with the scaling
+      return fmaxf(m0, m1);
+    };
+
+    float mb = -INFINITY;                                 // exponent base (lags the true max by < GAP), the same in both halves
+    float l = 0.f;                                        // sum over this warp's keys
+    // The first base is the maximum over the first TWO tiles (128 keys).  A weight at the base is 1 in bf16 and carries
+    // no rounding error; where the base lags, the row's largest weight carries up to 2^-8 of itself, and in a row that one
+    // key dominates that is the error of the output.  With one tile's maximum the attention of 130 slots and 64
+    // tokens was 2.2e-3 off 64 bits where it now is 2.0e-3, most of it the rounding of the result (queries of twice unit
+    // variance; the rounding of the weights alone: 1.3e-3 against 0.9e-3).
+    // It costs a CTA the wait for the second Q.K^T: 88.4 -> 90.8, 242 -> 254, 90.5 -> 95.5 and 131 -> 137 us at the four shapes above.
+    float ahead = -INFINITY;
+    if (NT > 1) {
+      uint32_t vis, v[32];
+      const int cls = visible(1, vis);
+      ahead = load_s(1, vis, cls, v);
+    }
+    for (int it = 0; it < NT; ++it) {
+      const uint32_t s_col = lane_addr + (uint32_t)(it & 1) * PF_BN;
+      uint32_t vis, v[32];
+      const int cls = visible(it, vis);
+      const float ms = fmaxf(load_s(it, vis, cls, v), ahead);
+      ahead = -INFINITY;
+      float mx = ms * p.scale_log2;                       // scale > 0: max commutes with the scaling
       // The other half of the row is in another warp.  Most tiles move no base: one barrier says so for the 32 rows (and
       // that both warps hold their part of S in registers, which P may then overwrite); else the maxima are exchanged.
       if (bar_pair_any(quarter, mx > mb + PF_RESCALE_GAP || (mb == -INFINITY && mx > -INFINITY))) {

@@ -33,6 +33,37 @@ def test_prefill_attention_at_tile_edges(Dh, H, Hkv, W, Me, Ms, norm, block, L):
     assert rel_err(ya, yb) < 8e-3
 
 
+@pytest.mark.parametrize("Dh", [64, 128])
+def test_prefill_attention_weight_of_the_dominating_key_is_exact(Dh):
+    """Two visible slots, one in each of the first two 64-key tiles, the second 2^6..2^8 times as heavy as the first, the same
+    value behind every visible key: whatever the weights, the output is that value.  The heavy key's weight must be the 1 that
+    bf16 holds exactly; taken against the first tile's maximum it is rounded by more than half a step of the value (keys
+    chosen so), and the output is the next bf16 value."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    W, L, v = 128, 8, 1.9921875                              # v: half a bf16 step is 2^-8, 0.196 % of it
+    s = torch.arange(0, 2000).mul(2.0 ** -5).to(torch.bfloat16).double().unique()     # candidate keys, query 8 in their place
+    w = torch.exp(s * 8.0 / Dh ** 0.5)
+    keep = (w > 2.0 ** 6) & (w < 2.0 ** 7.9) & ((w.float().to(torch.bfloat16).double() - w) / (w + 1) > 2.2e-3)
+    s = s[keep]
+    B = s.numel()
+    assert B >= 3
+    mod = CoDAGQALandmarkPerf2(embed_dim=2 * Dh, num_heads=2, num_kv_heads=1, window=W, num_landmarks_exact=0,
+                               num_landmarks_summary=0, head_norm_mode="identity").eval().to(torch.bfloat16).cuda()
+    st = mod.init_state(batch_size=B, device="cuda", dtype=torch.bfloat16)
+    st.v_buf.fill_(v)
+    for b in range(B):
+        heavy = 64 + 7 * b % 64
+        st.allowed[b, [5, heavy]] = True
+        st.k_buf[b, 0, heavy, 0] = s[b].float()
+    q, k, val = (torch.zeros(B, L, n * Dh, device="cuda", dtype=torch.bfloat16) for n in (2, 1, 1))
+    q[..., 0] = q[..., Dh] = 8.0
+    k[..., 0], val[:] = -100.0, v                            # the block's own keys weigh nothing
+    lam, out = torch.zeros(B, L, 2, device="cuda"), torch.empty_like(q)
+    mod._attend_block_tc(mod._cfg(B, torch.bfloat16, st), st, L, 0, L, q, q.clone(), lam, k, val, out)
+    assert mod.device_status() == 0
+    assert torch.equal(out, torch.full_like(out, v))
+
+
 @pytest.mark.parametrize("Dh", [32, 64, 128])
 @pytest.mark.parametrize("Lq,blk,Lbuf,used", [(1, False, 70, 0.5), (1, False, 200, 0.02), (2, True, 33, 0.0), (3, True, 40, 0.6),
                                               (8, True, 96, 1.0), (9, True, 31, 0.3), (65, True, 130, 0.1), (130, True, 5, 0.0)])
