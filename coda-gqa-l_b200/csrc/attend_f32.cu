@@ -1,8 +1,8 @@
 // Differential attention in single precision, register-tiled: head_dim 32, 64 or 128, 16-byte aligned rows.
 //
-// One CTA = one (state, query head, query tile); its four warps split the keys: warp w takes the 32-key tiles w, w+4,
+// One CTA = one (state, query head, query tile); its WARPS warps split the keys: warp w takes the 32-key tiles w, w+WARPS,
 // ... of the visible slots followed by the block's own tokens (causal), each with a running softmax of its own, and the
-// four partial results are merged once at the end (fixed order, no atomics).  The ROWS rows of a tile are the queries'
+// partial results are merged once at the end (fixed order, no atomics).  The ROWS rows of a tile are the queries'
 // signal vectors followed by their noise vectors, so both streams use every staged K/V element.  Per tile a warp
 // computes S as 4 row groups x 8 key groups of TM x 4 register tiles (K and Q read from shared memory as 16-byte
 // vectors along Dh), leaves P transposed in its own shared memory, and accumulates P.V as TM rows x Dh/8 columns per
@@ -11,15 +11,18 @@
 // Bound: FMA issue.  A row per warp and a key per lane (attend_generic) reads shared memory once per FMA and keeps
 // few warps in flight.
 // 256 queries of 8 heads over 384 slots + their own block, Dh 64: 219 -> 35 us.
-// The instance is chosen by the number of queries: 8 per CTA (TM = 4) for blocks; 2 (TM = 1) for decode steps, where
-// three rows in four of the larger tile would be padding.
+// The instance follows the call, not the batch (a state's result does not depend on its neighbours):
+// * queries per CTA: 8 (TM = 4) for blocks, 4 (TM = 2) and 2 (TM = 1) for calls of up to four and two, whose
+//   larger tile would be padding;
+// * warps: four, or as many as there are key tiles (one, two).  A warp without a tile still holds its buffers, and at Dh 128
+//   four warps' are a whole SM's: 800 heads of one query over 64 slots take 19.1 us with two warps, 46.1 with four (generic:
+//   34.7); over 32 slots 10.1 with one, 45.6 with four (19.0).
 #include "coda_common.cuh"
 #include "attend_f32.h"
 #include <type_traits>
 
 namespace {
 
-constexpr int AF_WARPS = 4;
 constexpr int AF_TK = 32;        // keys per warp tile
 
 __device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
@@ -30,7 +33,7 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int DH, int TM>
+template <int DH, int TM, int WARPS>
 struct AfLayout {
   static constexpr int ROWS = 4 * TM;          // rows of a tile, both streams
   static constexpr int BQ = ROWS / 2;          // queries of a tile
@@ -38,12 +41,12 @@ struct AfLayout {
   static constexpr int KS = DH + 4;            // different banks
   static constexpr int PS = ROWS + 4;
   static constexpr int WARP = AF_TK * KS + AF_TK * DH + AF_TK * PS;     // floats of one warp: K, V, P
-  static constexpr int FLOATS = ROWS * QS + AF_WARPS * WARP + 2 * AF_WARPS * ROWS;
+  static constexpr int FLOATS = ROWS * QS + WARPS * WARP + 2 * WARPS * ROWS;
 };
 
-template <int DH, int TM>
-__global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p) {
-  typedef AfLayout<DH, TM> Lay;
+template <int DH, int TM, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) attend_f32_kernel(AttnParams p) {
+  typedef AfLayout<DH, TM, WARPS> Lay;
   constexpr int ROWS = Lay::ROWS, BQ = Lay::BQ, QS = Lay::QS, KS = Lay::KS, PS = Lay::PS;
   constexpr int CH = DH / 4;                   // 16-byte chunks per row
   constexpr int NC = DH / 32;                  // 16-byte column chunks of the output per lane
@@ -55,8 +58,8 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
   float* Ks = Qs + ROWS * QS + warp * Lay::WARP;   // [TK][KS]
   float* Vs = Ks + AF_TK * KS;                 // [TK][DH]
   float* Ps = Vs + AF_TK * DH;                 // [TK][PS]
-  float* Ms = sm + ROWS * QS + AF_WARPS * Lay::WARP;   // [WARPS][ROWS] maxima, then sums
-  float* Ls = Ms + AF_WARPS * ROWS;
+  float* Ms = sm + ROWS * QS + WARPS * Lay::WARP;   // [WARPS][ROWS] maxima, then sums
+  float* Ls = Ms + WARPS * ROWS;
 
   const bool has_blk = p.kblk != nullptr;
   const int nblk_keys = has_blk ? min(q0 + BQ, p.Lq) : 0;
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
   auto key_ok = [&](int j) { return j < p.Lbuf ? (!p.mask_unused || al[j] != 0) : j < nkeys; };
   // the first tile at or after t (of this warp's) with such a key, and its mask
   auto next_tile = [&](int t, unsigned& bits) {
-    for (; t < ntiles; t += AF_WARPS) {
+    for (; t < ntiles; t += WARPS) {
       bits = __ballot_sync(0xffffffffu, key_ok(t * AF_TK + lane));
       if (bits != 0u) break;
     }
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
   unsigned bits = 0u;
   int t = next_tile(warp, bits);
   if (t < ntiles) { load(Ks, KS, kbase, kblk, p.kb_rs, t); load(Vs, DH, vbase, vblk, p.vb_rs, t); }
-  for (int c = tid; c < ROWS * CH; c += AF_WARPS * 32) {
+  for (int c = tid; c < ROWS * CH; c += WARPS * 32) {
     const int r = c / CH, cc = c % CH, q = q0 + (r % BQ);
     const float* src = r < BQ ? (const float*)p.q + (long long)b * p.q_bs + (long long)q * p.q_rs
                               : (const float*)p.qn + (long long)b * p.qn_bs + (long long)q * p.qn_rs;
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
     for (int c = 0; c < NC * 4; ++c) acc[i][c] = 0.f;
   }
   while (t < ntiles) {
-    const bool nok = t + AF_WARPS < ntiles && key_ok((t + AF_WARPS) * AF_TK + lane);   // (arrives under Q.K^T)
+    const bool nok = t + WARPS < ntiles && key_ok((t + WARPS) * AF_TK + lane);   // (arrives under Q.K^T)
     cp_wait<1>();                              // this tile's K (V is the younger group)
     __syncwarp();
     float s[TM][4];
@@ -131,9 +134,9 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
       }
     }
     __syncwarp();
-    int tn = t + AF_WARPS;
+    int tn = t + WARPS;
     unsigned nbits = __ballot_sync(0xffffffffu, nok);
-    if (nbits == 0u) tn = next_tile(tn + AF_WARPS, nbits);
+    if (nbits == 0u) tn = next_tile(tn + WARPS, nbits);
     if (tn < ntiles) load(Ks, KS, kbase, kblk, p.kb_rs, tn); else cp_commit();
     // visibility (the causal limit differs between the queries), running maximum, probabilities
 #pragma unroll
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
     const int r = rg * TM + i;
     float mm = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < AF_WARPS; ++w) mm = fmaxf(mm, Ms[w * ROWS + r]);
+    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, Ms[w * ROWS + r]);
     const float f = m[i] == -INFINITY ? 0.f : exp2f(m[i] - mm);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
   __syncthreads();
 
   // ---- epilogue: sig - lam*noise, optional RMSNorm over Dh (attention.py:463-464, primitives.py:23-27); a warp per query
-  for (int qi = warp; qi < BQ && q0 + qi < p.Lq; qi += AF_WARPS) {
+  for (int qi = warp; qi < BQ && q0 + qi < p.Lq; qi += WARPS) {
     const int row = q0 + qi;
     const float lam = p.lam[(long long)b * p.lam_bs + (long long)row * p.lam_rs + h];
     float il[2];
@@ -238,9 +241,9 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
       const int r = s * BQ + qi;
       float mm = -INFINITY, ll = 0.f;
 #pragma unroll
-      for (int w = 0; w < AF_WARPS; ++w) mm = fmaxf(mm, Ms[w * ROWS + r]);
+      for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, Ms[w * ROWS + r]);
 #pragma unroll
-      for (int w = 0; w < AF_WARPS; ++w) {
+      for (int w = 0; w < WARPS; ++w) {
         const float mw = Ms[w * ROWS + r];
         ll += mw == -INFINITY ? 0.f : Ls[w * ROWS + r] * exp2f(mw - mm);
       }
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
     for (int c = 0; c < NC; ++c) {
       float o[2] = {0.f, 0.f};
 #pragma unroll
-      for (int w = 0; w < AF_WARPS; ++w) {
+      for (int w = 0; w < WARPS; ++w) {
         const float* po = sm + ROWS * QS + w * Lay::WARP;
         o[0] += po[qi * DH + lane + 32 * c];
         o[1] += po[(BQ + qi) * DH + lane + 32 * c];
@@ -267,20 +270,28 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attend_f32_kernel(AttnParams p)
   }
 }
 
-template <int DH, int TM>
+template <int DH, int TM, int WARPS>
 int launch(const AttnParams& p, cudaStream_t s) {
-  typedef AfLayout<DH, TM> Lay;
+  typedef AfLayout<DH, TM, WARPS> Lay;
   static_assert(Lay::ROWS <= AF_TK, "partial rows are left in the K buffer");
   constexpr int bytes = Lay::FLOATS * 4;
   static coda_device_once once;
-  coda_on_first_use(once, [] { cudaFuncSetAttribute(attend_f32_kernel<DH, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
-  coda_launch_chained(attend_f32_kernel<DH, TM>, dim3((p.Lq + Lay::BQ - 1) / Lay::BQ, p.H, p.B), dim3(AF_WARPS * 32), bytes, s, 1, p);
+  coda_on_first_use(once, [] { cudaFuncSetAttribute(attend_f32_kernel<DH, TM, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+  coda_launch_chained(attend_f32_kernel<DH, TM, WARPS>, dim3((p.Lq + Lay::BQ - 1) / Lay::BQ, p.H, p.B), dim3(WARPS * 32), bytes, s, 1, p);
   CODA_CHECK_LAUNCH("attend (f32)");
   return CODA_OK;
 }
 
+template <int DH, int TM>
+int launch_warps(const AttnParams& p, cudaStream_t s) {
+  const int tiles = (p.Lbuf + (p.kblk != nullptr ? p.Lq : 0) + AF_TK - 1) / AF_TK;
+  return tiles <= 1 ? launch<DH, TM, 1>(p, s) : tiles <= 2 ? launch<DH, TM, 2>(p, s) : launch<DH, TM, 4>(p, s);
+}
+
 template <int DH>
-int launch_rows(const AttnParams& p, cudaStream_t s) { return p.Lq <= 2 ? launch<DH, 1>(p, s) : launch<DH, 4>(p, s); }
+int launch_rows(const AttnParams& p, cudaStream_t s) {
+  return p.Lq <= 2 ? launch_warps<DH, 1>(p, s) : p.Lq <= 4 ? launch_warps<DH, 2>(p, s) : launch_warps<DH, 4>(p, s);
+}
 
 }  // namespace
 

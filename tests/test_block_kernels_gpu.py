@@ -66,9 +66,10 @@ def test_prefill_attention_weight_of_the_dominating_key_is_exact(Dh):
 
 @pytest.mark.parametrize("Dh", [32, 64, 128])
 @pytest.mark.parametrize("Lq,blk,Lbuf,used", [(1, False, 70, 0.5), (1, False, 200, 0.02), (2, True, 33, 0.0), (3, True, 40, 0.6),
-                                              (8, True, 96, 1.0), (9, True, 31, 0.3), (65, True, 130, 0.1), (130, True, 5, 0.0)])
+                                              (8, True, 96, 1.0), (9, True, 31, 0.3), (65, True, 130, 0.1), (130, True, 5, 0.0),
+                                              (1, False, 20, 0.5), (4, True, 12, 0.5), (5, True, 27, 0.9), (4, True, 60, 0.7), (4, True, 100, 0.4)])
 def test_single_precision_attention(Dh, Lq, blk, Lbuf, used):
-    """The register-tiled fp32 kernel (both row counts per tile, keys split over four warps, tiles without a visible key)
+    """The register-tiled fp32 kernel (every row count per tile, keys split over one, two and four warps, tiles without a visible key)
     against the same attention in 64 bits; 32-bit sums over at most 260 keys."""
     from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
     H, Hkv, B = 4, 2, 2
