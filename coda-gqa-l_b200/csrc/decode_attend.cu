@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(128) decode_prep_kernel(DecodeParams p, const 
 // CTAs per SM: a plane is a chain (record, tiles, hand-over, merge) that the three roles overlap with the next plane's,
 // but where a plane holds few bytes (head_dim 64) the roles' own chains are longer than its tiles take to arrive, so
 // two CTAs share an SM there, each with half of the ring: 28.1 -> 23.4 us for 512 states x 3 heads of 192 slots.
-// (16 query rows do not fit half the registers, and calls with no more planes than SMs keep one CTA per SM, all its
-// registers and the whole ring.)
+// (16 query rows do not fit half the registers.)  Which calls gain is two_ctas()' matter, below.
 template <int DH, int NQ, bool APPEND, int CTAS>
 __global__ void __launch_bounds__(DA_THREADS, CTAS)
 decode_attend_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, DecodeParams p) {
@@ -747,13 +746,32 @@ int launch_decode_ctas(const CUtensorMap& km, const CUtensorMap& vm, DecodeParam
   return CODA_OK;
 }
 
+// Head_dim 64: two CTAs per SM, or one with the whole ring and all registers?  Planes per SM, slot tiles per plane, and
+// what a CTA does beside the attention decide; measured one against the other at 148 SMs, 31 plane counts from 150 to 2000, 192 to
+// 1016 slots, 1, 3 and 4 query heads per KV head, state cold in L2 (ratio: one CTA's time over two CTAs').
+// * No more planes than SMs: one (0.79 .. 1.0).
+// * Short planes: two.  Attention alone, up to 5 tiles: 1.0 .. 1.34.  With the new token's writing (its registers spill
+//   at two CTAs), up to 4 tiles: 1.0 .. 1.26 -- with one or two query heads, whose record takes the spilling warps
+//   nearly all their time, only from two planes per SM on (0.97 .. 1.02 below), up to 2 tiles 1.17 .. 1.37.
+// * Longer planes: up to 5/3 planes per SM (attention alone, up to 7 tiles: two) two CTAs spare a second round of which most SMs
+//   see nothing (1.0 .. 1.2).  From there to three per SM they leave a second round nearly as empty (0.85 .. 1.05).  Above three
+//   the attention alone is faster with two (1.03 .. 1.3); with the token's writing only up to 6 tiles (0.97 .. 1.15; 7 and
+//   more 0.85 .. 1.05).
+static bool two_ctas(long long planes, int num_sms, int tiles, int heads, bool append) {
+  if (planes <= num_sms) return false;
+  if (append && heads < 3) return tiles <= 2 || (tiles <= 4 && planes > 2 * num_sms);
+  if (tiles <= (append ? 4 : 5) || 3 * planes <= (!append && tiles <= 7 ? 6 : 5) * num_sms) return true;
+  return planes > 3 * num_sms && (!append || tiles <= 6);
+}
+
 template <int DH, int NQ, bool APPEND>
 int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, const DecodeParams& p, cudaStream_t s) {
   if constexpr (DH == 64 && NQ == 1) {
     static coda_device_once once;
     const int num_sms = coda_on_first_use(once, [] {});
     const bool fits = (DA_BUDGET / 2 - DecodeSmem<DH>(0, p.G, p.Lbuf).total - 1024) / (2 * DecodeSmem<DH>::TILE_BYTES) >= 2;
-    if (p.B * p.Hkv > num_sms && fits) return launch_decode_ctas<DH, NQ, APPEND, 2>(km, vm, p, s);
+    if (fits && two_ctas((long long)p.B * p.Hkv, num_sms, (p.Lbuf + DA_TILE - 1) / DA_TILE, p.G, APPEND))
+      return launch_decode_ctas<DH, NQ, APPEND, 2>(km, vm, p, s);
   }
   return launch_decode_ctas<DH, NQ, APPEND, 1>(km, vm, p, s);
 }

@@ -163,6 +163,11 @@ def test_block_routing_matches_oracle(monkeypatch, kw, Te, Ts, block, B):
     (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=700, num_landmarks_exact=140, num_landmarks_summary=60), 2),
     (dict(embed_dim=192, num_heads=3, num_kv_heads=3, window=32, num_landmarks_exact=32, num_landmarks_summary=32), 150),
     (dict(embed_dim=512, num_heads=8, num_kv_heads=1, window=33, num_landmarks_exact=5, num_landmarks_summary=90), 7),
+    # the attention's lines between one and two CTAs per SM: two short tiles, six tiles below and above three planes per SM, one query head
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=1, window=100, num_landmarks_exact=12, num_landmarks_summary=12), 160),
+    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 110),
+    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 155),
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 120),
 ])
 def test_batched_routing_head_dim_64(kw, B):
     """128-thread CTAs of the all-layers routing launch (more slots, stamps and cache chunks than threads) and two attention
