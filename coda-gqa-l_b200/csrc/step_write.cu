@@ -965,8 +965,7 @@ __global__ void __launch_bounds__(256) step_write_cluster_kernel(StepParams p) {
 // device array.  The routing of one layer is a latency chain that keeps an SM's resources while it waits; all
 // layers' chains side by side fill the machine and are bounded by memory bandwidth instead.
 // The chain is as long with 128 threads as with 256 and a CTA needs no more of them at Dh 64, so there twice as many
-// chains share an SM: 122 -> 86 us for 8 layers x 512 states x 3 heads.  As long as every chain is resident at once with 256
-// threads (five CTAs per SM) the wider CTA is the faster one (80 chains: 29.1 against 30.2 us per one-layer step).
+// chains share an SM: 122 -> 86 us for 8 layers x 512 states x 3 heads.  Which calls gain: fewer_rounds(), below.
 template <typename T, int DH, bool STAGE, int NCTA, int NT>
 __global__ void __launch_bounds__(NT, NCTA) step_route_batched_kernel(const StepParams* __restrict__ layers) {
   __shared__ StepParams sp;
@@ -1176,6 +1175,36 @@ extern "C" int coda_b200_step_route_plan(const coda_layer_cfg* cfg, const coda_s
   return CODA_OK;
 }
 
+template <int DH, bool STAGE, int NCTA, int NT>
+static cudaError_t route_batched_launch(cudaLaunchConfig_t& lc, const StepParams* plan) {
+  lc.blockDim = dim3(NT, 1, 1);
+  return cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, DH, STAGE, NCTA, NT>, plan);
+}
+// Clusters of this launch that the device holds at once (the shared memory and the cluster size of the call included)
+template <int DH, bool STAGE, int NCTA, int NT>
+static long long route_batched_resident(cudaLaunchConfig_t lc) {
+  lc.blockDim = dim3(NT, 1, 1);
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, step_route_batched_kernel<bf16, DH, STAGE, NCTA, NT>, &lc) != cudaSuccess) { cudaGetLastError(); return 0; }
+  return n;
+}
+// Head_dim 64: does the launch go through in so many fewer rounds with 128 threads per CTA that they are the better choice?  A
+// round of twice as many chains takes longer; by how much depends on where the caches are read.  Measured at 400 to 4800
+// chains, 1 to 8 KV heads (ratio: 256 threads' time over 128 threads'):
+// * caches staged in shared memory: any round less pays (1.06 .. 1.56); as many rounds, e.g. 1200 .. 1400 chains of 64 + 64 slots,
+//   0.89 .. 1.07;
+// * caches read by the scoring threads: two rounds for one, or five for three, pay (1.02 .. 1.22); three for two do not (0.93 ..
+//   1.03: 1200 chains of 255 + 100 slots 33.0 against 35.4 us).
+template <bool STAGE>
+static bool fewer_rounds(const cudaLaunchConfig_t& lc) {
+  const long long wide = STAGE ? route_batched_resident<64, true, 5, 256>(lc) : route_batched_resident<64, false, 4, 256>(lc);
+  const long long narrow = STAGE ? route_batched_resident<64, true, 10, 128>(lc) : route_batched_resident<64, false, 8, 128>(lc);
+  if (wide <= 0 || narrow <= 0) return false;
+  const long long clusters = (long long)lc.gridDim.y * lc.gridDim.z;         // one per state and layer
+  const long long rw = (clusters + wide - 1) / wide, rn = (clusters + narrow - 1) / narrow;
+  return STAGE ? rw > rn : 5 * rw >= 8 * rn;
+}
+
 extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const void* plan_dev, int32_t n_layers,
                                             coda_stream_t stream) {
   CODA_REQUIRE(coda_b200_step_write_fused_supported(cfg), CODA_ERR_ARG,
@@ -1185,10 +1214,6 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
   const int MM = cfg->Me + cfg->Ms;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(cfg->Hkv, cfg->B, n_layers);
-  static coda_device_once once;
-  const int num_sms = coda_on_first_use(once, [] {});
-  const bool narrow = cfg->Dh == 64 && (long long)cfg->Hkv * cfg->B * n_layers > 5LL * num_sms;      // 128-thread CTAs, see the kernel
-  lc.blockDim = dim3(narrow ? 128 : 256, 1, 1);
   lc.dynamicSmemBytes = sizeof(float) * ((size_t)cfg->Hkv * MM + MM) + 8 + 8 * (size_t)cfg->Me + (size_t)(cfg->W + MM) + 16;
   lc.stream = (cudaStream_t)stream;
   cudaLaunchAttribute at[1];
@@ -1204,13 +1229,11 @@ extern "C" int coda_b200_step_route_batched(const coda_layer_cfg* cfg, const voi
   if (stage) {
     lc.dynamicSmemBytes += 16 + stage_bytes;
     // five CTAs per SM measured best at the 7B shape (4: 122 us, 5: 111 us, 6: 114 us for 32 layers x 32 states)
-    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, true, 5, 256>, plan)
-        : narrow         ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 10, 128>, plan)
-                         : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, true, 5, 256>, plan);
+    e = cfg->Dh == 128 ? route_batched_launch<128, true, 5, 256>(lc, plan)
+        : fewer_rounds<true>(lc) ? route_batched_launch<64, true, 10, 128>(lc, plan) : route_batched_launch<64, true, 5, 256>(lc, plan);
   } else {
-    e = cfg->Dh == 128 ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 128, false, 4, 256>, plan)
-        : narrow         ? cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 8, 128>, plan)
-                         : cudaLaunchKernelEx(&lc, step_route_batched_kernel<bf16, 64, false, 4, 256>, plan);
+    e = cfg->Dh == 128 ? route_batched_launch<128, false, 4, 256>(lc, plan)
+        : fewer_rounds<false>(lc) ? route_batched_launch<64, false, 8, 128>(lc, plan) : route_batched_launch<64, false, 4, 256>(lc, plan);
   }
   if (e != cudaSuccess) { coda_set_error("step_route_batched: %s", cudaGetErrorString(e)); return CODA_ERR_LAUNCH; }
   return CODA_OK;
