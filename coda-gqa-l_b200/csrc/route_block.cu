@@ -112,8 +112,9 @@ __device__ __forceinline__ void route_score_bank(const RouteParams& p, int b, bo
               else
                 for (int i = 0; i < KRUN_A; ++i) if (k0 + kq0 + i < n) x[i] = El<T>::ld(row + k0 + kq0 + i);
               const float dn = den[r * Hkv + h];
+              // (the division out of line: inlined, the reciprocal form made this loop 4 % slower, 98 -> 102 us for 16 states of 16 heads)
 #pragma unroll
-              for (int i = 0; i < KRUN_A; ++i) x[i] = t_div<T>(x[i], dn);
+              for (int i = 0; i < KRUN_A; ++i) x[i] = El<T>::rnd(div_rn_call(x[i], dn));
             }
 #pragma unroll
             for (int i = 0; i < KRUN_A; ++i) As[(kq0 + i) * ROWS + r] = x[i];
