@@ -247,3 +247,31 @@ def test_routing_caches_of_a_fresh_state(dtype, H, Hkv, Dh, Me, Ms):
             if got is not None:
                 assert torch.allclose(got.double(), F.normalize(src, dim=-1, eps=1e-6).double(), rtol=ulp, atol=0)
 
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("interleaved,Dh,H,Hkv", [(True, 128, 3, 1), (False, 64, 3, 3), (True, 24, 2, 1), (False, 32, 4, 2)])
+@pytest.mark.parametrize("B,L", [(2, 1), (1, 1184), (70, 37), (331, 37), (5, 1201)])
+def test_projection_postprocessing_tiles(dtype, interleaved, Dh, H, Hkv, B, L):
+    """The vector kernel's tiles of one token, of several positions, of positions and states, and their remainders, against the
+    element-wise kernel (rows that start one element off a 16-byte boundary): the same operations, so the same bits."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    torch.manual_seed(1)
+    mod = CoDAGQALandmarkPerf2(embed_dim=H * Dh, num_heads=H, num_kv_heads=Hkv, window=16, num_landmarks_exact=4,
+                               num_landmarks_summary=4, rope_interleaved=interleaved, rope_base=1e6).eval()
+    randomize_weights(mod, 2)
+    mod = mod.to(dtype).cuda()
+    cfg = mod._cfg(B, dtype, mod.init_state(batch_size=B, device="cuda", dtype=dtype))
+    nq, nk = H * Dh, Hkv * Dh
+    n = nq + nk + H + 1
+    src = torch.randn(B, L, n, generator=torch.Generator("cuda").manual_seed(4), device="cuda").to(dtype)
+    outs = []
+    for shift in (0, 1):
+        y = torch.zeros(B, L, (n + 16) // 8 * 8, device="cuda", dtype=dtype)
+        y[..., shift:shift + n] = src
+        q, k, lam_logit, gate_logit = y[..., shift:shift + n].split([nq, nk, H, 1], -1)
+        qn, lam, gate = mod._prep(cfg, L, 1000, q, k, lam_logit, gate_logit, True)
+        outs.append((q, k, qn, lam, gate))
+    for a, b, name in zip(*outs, ("q", "k", "q_noise", "lambda", "gate")):
+        assert torch.equal(a, b), name
+    assert not torch.equal(outs[0][0], src[..., :nq]) and not torch.equal(outs[0][0], outs[0][2])
