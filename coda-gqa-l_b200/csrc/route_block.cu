@@ -441,8 +441,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
   const int te = (Me > 0) ? p.te : 0, ts = (Ms > 0) ? p.ts : 0, tmax = te > ts ? te : ts;
   typedef topk_order::Item<long long> It64;
   It64* lruq = reinterpret_cast<It64*>(smraw);                       // [Me]
-  long long* s_last = reinterpret_cast<long long*>(lruq + (Me > 0 ? Me : 1));   // [Me]
-  float* c_g = reinterpret_cast<float*>(s_last + (Me > 0 ? Me : 1)); // [tmax] gates
+  float* c_g = reinterpret_cast<float*>(lruq + (Me > 0 ? Me : 1));   // [tmax] gates
   float* x_best = c_g + (tmax > 0 ? tmax : 1);                       // [te]
   float* w_s = x_best + (te > 0 ? te : 1);                           // [ts] summary weights
   int* c_e = reinterpret_cast<int*>(w_s + (ts > 0 ? ts : 1));        // [tmax] evicted index
@@ -470,7 +469,6 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
     const bool used = __ldcg(al + W + m) != 0;
     const long long stamp = __ldcg(last + m);
     s_used[m] = used;
-    s_last[m] = stamp;
     lruq[m].v = (used && m < Ae) ? stamp : -(1LL << 62);
     lruq[m].i = m;
     n_first[m] = 0x7fffffff; n_e[m] = -1;
@@ -523,9 +521,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_decide_kernel(RouteParams p)
       __syncwarp();
       // stamps: per slot the largest position among touching candidates replaces the old stamp (:682-697)
       for (int m = lane; m < Me; m += 32) {
-        if (n_e[m] < 0) continue;
-        const long long stamp = p.pos_first + n_e[m];
-        if (stamp != s_last[m]) last[m] = stamp;
+        if (n_e[m] >= 0) last[m] = p.pos_first + n_e[m];
       }
     }
     return;
@@ -883,7 +879,7 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
     }
     const int tmax = p.te > p.ts ? p.te : p.ts;
     const size_t me1 = c.Me > 0 ? c.Me : 1;
-    const size_t smem2 = me1 * (16 + 8 + 4 + 4 + 4) + 4 * ((size_t)2 * (tmax + 1) + 2 * (size_t)(p.te + 1) + 2 * (size_t)(p.ts + 1) +
+    const size_t smem2 = me1 * (16 + 4 + 4 + 4) + 4 * ((size_t)2 * (tmax + 1) + 2 * (size_t)(p.te + 1) + 2 * (size_t)(p.ts + 1) +
                          (size_t)c.Ms + 2) + c.Me + c.Ms + 64;
     CODA_REQUIRE(smem2 <= 200 * 1024, CODA_ERR_LIMIT, "route_block: decision stage needs %zu bytes of shared memory", smem2);
     if (smem2 > 48 * 1024) cudaFuncSetAttribute(route_decide_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);

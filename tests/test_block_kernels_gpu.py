@@ -144,6 +144,8 @@ def test_single_precision_attention_keeps_later_tokens_out(Dh, bad):
     # rows above 256 elements: four warps per slot; one KV head: no cluster
     (dict(num_heads=8, num_kv_heads=8, embed_dim=512, num_landmarks_exact=12, num_landmarks_summary=1), 5, 64, 70, 1),
     (dict(num_heads=2, num_kv_heads=1, embed_dim=128, num_landmarks_exact=1, num_landmarks_summary=3), 8, 64, 64, 2),
+    # as many exact slots as the decisions' shared memory holds (33 bytes each were enough for 6000)
+    (dict(num_heads=2, num_kv_heads=2, embed_dim=64, num_landmarks_exact=6000, num_landmarks_summary=4), 8, 64, 50, 1),
     # head_dim 20 and 12: chunks that straddle heads and the phase-safe half
     (dict(num_heads=4, num_kv_heads=2, embed_dim=80, num_landmarks_exact=16, num_landmarks_summary=16), 8, 64, 40, 2),
     (dict(num_heads=4, num_kv_heads=4, embed_dim=48, num_landmarks_exact=5, num_landmarks_summary=7), 3, 9, 33, 2),
