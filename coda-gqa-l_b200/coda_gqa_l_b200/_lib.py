@@ -13,6 +13,7 @@ LIB_PATH = os.path.join(_HERE, "libcoda_b200.so")
 
 CODA_F32, CODA_BF16 = 0, 1
 CODA_EVENT_WORDS = 16   # int32 words per state in the routing-event record (coda_b200.h)
+CODA_CACHE_WRITTEN = -16   # step_layer: an error at or below it came after the cache write (coda_b200.h)
 
 
 class LayerCfg(C.Structure):

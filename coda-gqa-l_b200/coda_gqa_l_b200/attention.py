@@ -685,9 +685,10 @@ class CoDAGQALandmarkPerf2(nn.Module):
                                               RingPos(st.pos, st.recent_idx, st.recent_filled, None), xp, rp_ or None,
                                               ws.data_ptr(), y.data_ptr(), self._decode_records(cfg, dev).data_ptr(),
                                               self._status_word(dev).data_ptr(), _stream(dev))
+                if rc == 0 or rc <= _lib.CODA_CACHE_WRITTEN:      # (the token is in the ring, whatever came after)
+                    self.advance_host_scalars(st)
                 if rc:
                     check(rc, "coda_b200_step_layer")
-                self.advance_host_scalars(st)
                 return y
         y = None
         if self.use_skinny_gemm_kernel:

@@ -138,5 +138,6 @@ extern "C" int coda_b200_step_layer(const coda_step_layer* l, const coda_layer_c
                                    l->eta_logit, proj, l->npad, proj + l->off_lam, l->npad, l->cos_theta, l->sin_theta, qrec,
                                    l->norm_w, heads, l->n_heads_out, status, stream);
   if (rc != CODA_OK) return rc;
-  return coda_b200_skinny_gemm(heads, cfg->B, l->n_heads_out, l->w_out, l->n_out, residual, l->n_out, y, l->n_out, status, stream);
+  rc = coda_b200_skinny_gemm(heads, cfg->B, l->n_heads_out, l->w_out, l->n_out, residual, l->n_out, y, l->n_out, status, stream);
+  return rc == CODA_OK ? CODA_OK : CODA_CACHE_WRITTEN + rc;
 }

@@ -37,7 +37,8 @@ enum {
   CODA_OK = 0,
   CODA_ERR_ARG = -1,      /* bad size / null pointer / unsupported combination */
   CODA_ERR_LAUNCH = -2,   /* the CUDA runtime refused the launch */
-  CODA_ERR_LIMIT = -3     /* a documented size limit was exceeded */
+  CODA_ERR_LIMIT = -3,    /* a documented size limit was exceeded */
+  CODA_CACHE_WRITTEN = -16 /* coda_b200_step_layer: added to the code of an error that came after the cache write */
 };
 
 /* Hyper-parameters of one layer; mirrors the constructor arguments of upstream
@@ -261,7 +262,8 @@ typedef struct coda_step_layer {
   int64_t off_k, off_v, off_lam, off_gate;
 } coda_step_layer;
 /* x [B][embed], residual [B][n_out] or null, y [B][n_out]; ws: B * (npad + n_heads_out) elements (projection rows, then head
- * outputs), 16-byte aligned, npad a multiple of 8. */
+ * outputs), 16-byte aligned, npad a multiple of 8.  Where the output projection fails the step's token is in the ring all the
+ * same: the code is then CODA_CACHE_WRITTEN + code, and the caller's ring scalars have to advance. */
 int coda_b200_step_layer(const coda_step_layer* layer, const coda_layer_cfg* cfg, const coda_state_ptrs* st, coda_ring_pos rp,
                          const void* x, const void* residual, void* ws, void* y, void* qrec, int32_t* status,
                          coda_stream_t stream);

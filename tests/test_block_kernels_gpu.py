@@ -277,3 +277,27 @@ def test_projection_postprocessing_tiles(dtype, interleaved, Dh, H, Hkv, B, L):
     for a, b, name in zip(*outs, ("q", "k", "q_noise", "lambda", "gate")):
         assert torch.equal(a, b), name
     assert not torch.equal(outs[0][0], src[..., :nq]) and not torch.equal(outs[0][0], outs[0][2])
+
+
+def test_step_whose_output_projection_is_refused_keeps_its_token():
+    """The one-call step writes the cache before the output projection: where that is refused (here by a width the GEMM does not
+    take, on the host), the error is raised and the ring scalars tell that the token is in, as when the calls were separate."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, _deep_copy_state
+    torch.manual_seed(2)
+    mod = CoDAGQALandmarkPerf2(embed_dim=256, num_heads=4, num_kv_heads=2, window=6, num_landmarks_exact=4,
+                               num_landmarks_summary=4).eval().to(torch.bfloat16).cuda()
+    x = torch.randn(12, 2, 1, 256, device="cuda", dtype=torch.bfloat16)
+    st = mod.init_state(batch_size=2, device="cuda", dtype=torch.bfloat16)
+    for t in range(10):
+        mod.step(x[t], st)
+    twin = _deep_copy_state(st)
+    mod.step(x[10], twin)
+    bd = mod._decode_bundle(x.device, x.dtype)
+    assert mod._one_call_ok(bd, 2)
+    bd["layer"].n_out = 100
+    with pytest.raises(RuntimeError, match="skinny_gemm"):
+        mod.step(x[10], st)
+    bd["layer"].n_out = bd["n_out"]
+    assert (st.pos, st.recent_idx, st.recent_filled) == (twin.pos, twin.recent_idx, twin.recent_filled)
+    ya, yb = mod.step(x[11], st)[0], mod.step(x[11], twin)[0]
+    assert torch.equal(ya, yb) and torch.equal(st.k_buf, twin.k_buf) and torch.equal(st.v_buf, twin.v_buf)
