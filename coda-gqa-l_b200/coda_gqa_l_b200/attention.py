@@ -254,8 +254,9 @@ class CoDAGQALandmarkPerf2(nn.Module):
             raise ValueError("mem_init must be 'zeros' or 'random_normal'")
         st.active_exact = self.Me_min if Me > 0 else 0
         st.active_summary = self.Ms_min if Ms > 0 else 0
-        if st.k_buf.is_cuda and st.k_buf.device.index == torch.cuda.current_device() and 0 < B <= 65535:
-            # both routing caches in one launch
+        plain = not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+        if plain and st.k_buf.is_cuda and st.k_buf.device.index == torch.cuda.current_device() and 0 < B <= 65535:
+            # both routing caches in one launch; a tracer or a dispatch mode (fake tensors) sees tensor operations
             cfg = LayerCfg(B=B, H=self.num_heads, Hkv=self.num_kv_heads, Dh=self.head_dim, W=W, Me=Me, Ms=Ms, dtype=_DT[dtype])
             check(lib.coda_b200_bank_norms(C.byref(cfg), C.byref(self._ptrs(st)), _stream(st.k_buf.device)), "coda_b200_bank_norms")
         else:

@@ -233,3 +233,28 @@ def test_quotient_of_bf16_values_rounds_the_same_from_an_approximate_reciprocal(
     want = q.to(torch.float32).to(torch.bfloat16)
     for eps in (-2.0 ** -21, 2.0 ** -21):
         assert torch.equal((q * (1 + eps)).to(torch.float32).to(torch.bfloat16), want)
+
+
+def test_fresh_state_under_a_dispatch_mode_is_made_of_tensor_operations():
+    """Shapes and memory of a CUDA state can be planned with fake tensors, on a machine without a GPU too, and a tracer sees every
+    write: no kernel is launched past the dispatcher."""
+    from torch._subclasses.fake_tensor import FakeTensor, FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    kw = dict(embed_dim=128, num_heads=4, num_kv_heads=2, window=8, num_landmarks_exact=4, num_landmarks_summary=6)
+    with FakeTensorMode():
+        layer = CoDAGQALandmarkPerf2(**kw).eval()
+        for dtype in (torch.float32, torch.bfloat16):
+            st = layer.init_state(batch_size=3, device="cuda", dtype=dtype)
+            assert isinstance(st.k_buf, FakeTensor) and st.k_buf.device.type == "cuda"
+            assert st._exact_v_norm.shape == (3, 2, 4, 32) and st._sum_lf_k_norm.shape == (3, 2, 6, 16)
+
+    seen = []
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Log():
+        CoDAGQALandmarkPerf2(**kw).eval().init_state(batch_size=1, device="cpu", dtype=torch.float32)
+    assert sum(name.startswith("aten.copy_") for name in seen) >= 2
