@@ -141,7 +141,7 @@ def test_single_precision_attention_keeps_later_tokens_out(Dh, bad):
     (dict(num_heads=4, num_kv_heads=2, embed_dim=128, num_landmarks_exact=40, num_landmarks_summary=33), 40, 70, 96, 2),
     (dict(num_heads=3, num_kv_heads=3, embed_dim=192, num_landmarks_exact=70, num_landmarks_summary=100), 33, 90, 100, 2),
     (dict(num_heads=2, num_kv_heads=2, embed_dim=256, num_landmarks_exact=8, num_landmarks_summary=32), 8, 64, 48, 3),
-    # rows above 256 elements: four warps per slot; one KV head: no cluster
+    # rows above 256 elements: eight warps per slot; one KV head: no cluster
     (dict(num_heads=8, num_kv_heads=8, embed_dim=512, num_landmarks_exact=12, num_landmarks_summary=1), 5, 64, 70, 1),
     (dict(num_heads=2, num_kv_heads=1, embed_dim=128, num_landmarks_exact=1, num_landmarks_summary=3), 8, 64, 64, 2),
     # as many exact slots as the decisions' shared memory holds (33 bytes each were enough for 6000)
@@ -161,19 +161,27 @@ def test_block_routing_matches_oracle(monkeypatch, kw, Te, Ts, block, B):
     _run("block_routing", check_golden=False)
 
 
-@pytest.mark.parametrize("kw,B", [
-    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=700, num_landmarks_exact=140, num_landmarks_summary=60), 2),
-    (dict(embed_dim=192, num_heads=3, num_kv_heads=3, window=32, num_landmarks_exact=32, num_landmarks_summary=32), 150),
-    (dict(embed_dim=512, num_heads=8, num_kv_heads=1, window=33, num_landmarks_exact=5, num_landmarks_summary=90), 7),
+@pytest.mark.parametrize("kw,B,narrow", [
+    # 128-thread CTAs: more slots, stamps and cache chunks than threads, caches staged; the same unstaged (more than 30 KB); few of each
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=700, num_landmarks_exact=140, num_landmarks_summary=60), 100, True),
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=64, num_landmarks_exact=200, num_landmarks_summary=100), 100, True),
+    (dict(embed_dim=192, num_heads=3, num_kv_heads=3, window=32, num_landmarks_exact=32, num_landmarks_summary=32), 150, True),
+    # 256-thread CTAs: the same, and one KV head
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=700, num_landmarks_exact=140, num_landmarks_summary=60), 2, False),
+    (dict(embed_dim=512, num_heads=8, num_kv_heads=1, window=33, num_landmarks_exact=5, num_landmarks_summary=90), 7, False),
     # the attention's lines between one and two CTAs per SM: two short tiles, six tiles below and above three planes per SM, one query head
-    (dict(embed_dim=256, num_heads=4, num_kv_heads=1, window=100, num_landmarks_exact=12, num_landmarks_summary=12), 160),
-    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 110),
-    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 155),
-    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 120),
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=1, window=100, num_landmarks_exact=12, num_landmarks_summary=12), 160, False),
+    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 95, False),
+    (dict(embed_dim=576, num_heads=9, num_kv_heads=3, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 155, True),
+    (dict(embed_dim=256, num_heads=4, num_kv_heads=4, window=300, num_landmarks_exact=40, num_landmarks_summary=40), 120, True),
 ])
-def test_batched_routing_head_dim_64(kw, B):
-    """128-thread CTAs of the all-layers routing launch (more slots, stamps and cache chunks than threads) and two attention
+def test_batched_routing_head_dim_64(kw, B, narrow):
+    """The all-layers routing launch with 128 and with 256 threads per CTA and the token-writing attention with one and with two
     CTAs per SM, through the captured step against eager steps: the same bits in both banks."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    chains = 2 * B * kw["num_kv_heads"]
+    # 256-thread CTAs fit an SM four or five times, 128-thread ones at least 6.6 times: two rounds against one, or one round of either
+    assert 5 * sms < chains <= 6.6 * sms if narrow else chains <= 4 * sms
     from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, CoDAStack, _deep_copy_state
     torch.manual_seed(5)
     layers = [CoDAGQALandmarkPerf2(**kw).eval() for _ in range(2)]
@@ -301,3 +309,95 @@ def test_step_whose_output_projection_is_refused_keeps_its_token():
     assert (st.pos, st.recent_idx, st.recent_filled) == (twin.pos, twin.recent_idx, twin.recent_filled)
     ya, yb = mod.step(x[11], st)[0], mod.step(x[11], twin)[0]
     assert torch.equal(ya, yb) and torch.equal(st.k_buf, twin.k_buf) and torch.equal(st.v_buf, twin.v_buf)
+
+
+def test_quotients_of_bf16_values_are_the_divisions():
+    """The device's bf16 quotient from an approximate reciprocal, seen through the unit vectors of a fresh state's slots: a row
+    holds one value b and values 2^-12 as large, so that its norm rounds to b exactly; every pair of significands, both signs,
+    with b from 2^-12 to 2^60, and rows below the smallest denominator (1e-6), down to subnormal values; equal bits."""
+    import ctypes as C
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, _lib as lib
+    Dh, Me = 128, 256
+    mod = CoDAGQALandmarkPerf2(embed_dim=Dh, num_heads=1, num_kv_heads=1, window=4, num_landmarks_exact=Me,
+                               num_landmarks_summary=0).eval().to(torch.bfloat16).cuda()
+    scales = [0, -12, 20, 60, -22, -60, -100, -118]
+    st = mod.init_state(batch_size=len(scales), device="cuda", dtype=torch.bfloat16, mem_init="zeros")
+    sig = 1.0 + torch.arange(128, device="cuda", dtype=torch.float64) / 128
+    rows = torch.empty(Me, Dh, device="cuda", dtype=torch.float64)     # row 2 i + j: b = sig[i], the others sig[j:j + 127]
+    rows[:, 0] = sig.repeat_interleave(2)
+    for j in range(2):
+        rows[j::2, 1:] = sig[j:j + 127] * 2.0 ** -12 * torch.tensor([1.0, -1.0], device="cuda").repeat(64)[:127]
+    for b, e in enumerate(scales):
+        st.v_buf[b, 0, 4:] = (rows * 2.0 ** e).to(torch.bfloat16)
+    x = st.v_buf[:, 0, 4:].clone()
+    ptrs = mod._ptrs(st)
+    lib.check(lib.lib.coda_b200_bank_norms(C.byref(mod._cfg(len(scales), torch.bfloat16, st)), C.byref(ptrs),
+                                           torch.cuda.current_stream().cuda_stream), "bank_norms")
+    smallest = torch.tensor(1e-6).to(torch.bfloat16).float().cuda()
+    for b, e in enumerate(scales):
+        den = torch.maximum(x[b, :, :1].float(), smallest)
+        assert torch.equal(st._exact_v_norm[b, 0], (x[b].float() / den).to(torch.bfloat16)), e
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("Lbuf,blk,scale", [(130, 64, 2.0), (384, 256, 0.5), (200, 333, 2.0), (768, 65, 6.0), (70, 1, 2.0)])
+def test_prefill_attention_error_against_64_bits(Dh, Lbuf, blk, scale):
+    """bf16 weights and a bf16 result, everything else in 32 bits: each weight off by at most 2^-8 of itself (and 1e-4 where its
+    exponential is a polynomial; 2^-16 for 32-bit sums), the result rounded once.  Bound per element, from the absolute values."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2
+    H, Hkv, B = 4, 2, 2
+    mod = CoDAGQALandmarkPerf2(embed_dim=H * Dh, num_heads=H, num_kv_heads=Hkv, window=Lbuf, num_landmarks_exact=0,
+                               num_landmarks_summary=0, head_norm_mode="identity").eval().to(torch.bfloat16).cuda()
+    st = mod.init_state(batch_size=B, device="cuda", dtype=torch.bfloat16)
+    g = torch.Generator("cuda").manual_seed(Dh + Lbuf + blk)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    st.k_buf.copy_(rnd(*st.k_buf.shape))
+    st.v_buf.copy_(rnd(*st.v_buf.shape))
+    st.allowed.copy_(torch.rand(B, Lbuf, generator=g, device="cuda") < 0.8)
+    q, qn, k, v = scale * rnd(B, blk, H * Dh), scale * rnd(B, blk, H * Dh), rnd(B, blk, Hkv * Dh), rnd(B, blk, Hkv * Dh)
+    lam = torch.rand(B, blk, H, generator=g, device="cuda").to(torch.bfloat16).float()
+    out = torch.full((B, blk, H * Dh), float("nan"), device="cuda", dtype=torch.bfloat16)
+    mod._attend_block_tc(mod._cfg(B, torch.bfloat16, st), st, blk, 0, blk, q, qn, lam, k, v, out)
+    assert mod.device_status() == 0
+
+    heads = lambda t, n: t.double().view(B, blk, n, Dh).transpose(1, 2)  # noqa: E731
+    keys = torch.cat([st.k_buf.double(), heads(k, Hkv)], 2).repeat_interleave(H // Hkv, 1)
+    vals = torch.cat([st.v_buf.double(), heads(v, Hkv)], 2).repeat_interleave(H // Hkv, 1)
+    vis = torch.cat([st.allowed.bool()[:, None].expand(B, blk, Lbuf),
+                     torch.ones(blk, blk, device="cuda").tril().bool().expand(B, blk, blk)], 2)[:, None]
+    w = [torch.softmax((heads(x, H) @ keys.transpose(2, 3) / Dh ** 0.5).masked_fill(~vis, float("-inf")), -1) for x in (q, qn)]
+    lam = lam.double().transpose(1, 2)[..., None]
+    want = w[0] @ vals - lam * (w[1] @ vals)
+    bound = (2.0 ** -8 + 1e-4 + 2.0 ** -16) * (w[0] @ vals.abs() + lam * (w[1] @ vals.abs())) + 2.0 ** -8 * want.abs()
+    err = (heads(out, H) - want).abs()
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("Dh,dtype", [(64, torch.bfloat16), (128, torch.bfloat16), (64, torch.float32), (20, torch.bfloat16)])
+def test_prefill_replayed_from_a_graph(Dh, dtype):
+    """The chained launches of a prefill's blocks captured and replayed: the bits of the plain call in the output and the state."""
+    from coda_gqa_l_b200 import CoDAGQALandmarkPerf2, _deep_copy_state
+    torch.manual_seed(5)
+    mod = CoDAGQALandmarkPerf2(embed_dim=4 * Dh, num_heads=4, num_kv_heads=2, window=96, num_landmarks_exact=16,
+                               num_landmarks_summary=16).eval()
+    randomize_weights(mod, 3)
+    mod = mod.to(dtype).cuda()
+    x = orc.mixture_inputs(3, 400, 4 * Dh, centroids=16, sigma=0.3, seed=5, dtype=dtype).cuda()
+    st = mod.init_state(batch_size=3, device="cuda", dtype=dtype)
+    mod.prefill_chunked(x[:, :200].contiguous(), st, block_size=64)
+    rest = x[:, 200:].contiguous()
+    twin, warm = _deep_copy_state(st), _deep_copy_state(st)
+    want, twin = mod.prefill_chunked(rest, twin, block_size=64)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        mod.prefill_chunked(rest, warm, block_size=64)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y, st = mod.prefill_chunked(rest, st, block_size=64)
+    graph.replay()
+    assert torch.equal(y, want) and (st.pos, st.recent_idx, st.recent_filled) == (twin.pos, twin.recent_idx, twin.recent_filled)
+    for f in ("k_buf", "v_buf", "allowed", "g_recent", "mem_last_exact", "_exact_v_norm", "_sum_lf_k_norm"):
+        assert torch.equal(getattr(st, f), getattr(twin, f)), f
+    assert mod.device_status() == 0

@@ -224,8 +224,9 @@ def test_captured_step_key_sees_every_way_a_parameter_can_change():
 
 
 def test_quotient_of_bf16_values_rounds_the_same_from_an_approximate_reciprocal():
-    """The device code rounds a * (1 / b) instead of a / b to bf16: every pair of significands, the product perturbed by
-    twice the error it can have (a reciprocal good to an ulp and one rounding: below 2^-22), rounds as the quotient does."""
+    """The argument behind the device's bf16 quotient, not the device's code (a GPU test compares that): a * (1 / b) rounds to bf16
+    as a / b does for every pair of significands, the product perturbed by twice the error it can have (a reciprocal good
+    to an ulp and one rounding: below 2^-22)."""
     import torch
     a = torch.arange(128, 256, dtype=torch.float64)[:, None]
     b = torch.arange(128, 256, dtype=torch.float64)[None, :]
