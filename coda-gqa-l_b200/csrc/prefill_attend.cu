@@ -146,10 +146,11 @@ __device__ __forceinline__ uint64_t add2_rm(uint64_t a, uint64_t b) {
   asm("add.rm.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// 2^x for a pair of arguments on the FMA / integer pipes (x = n + f, n = floor(x) left in the low mantissa bits
-// by a round-down add of 1.5 * 2^23; 2^f by a cubic, relative error < 1e-4, far below the bf16 rounding of P;
-// n added into the exponent field).  The special-function unit delivers one warp of exponentials per 8 cycles
-// per scheduler; a third of the exponentials go this way so that neither pipe bounds the softmax.
+// 2^x for a pair of arguments on the FMA / integer pipes: x = n + f, n = floor(x) left in the low mantissa bits by a
+// round-down add of 1.5 * 2^23, 2^f by a cubic, n added into the exponent field.  The cubic is the one with p(0) = 1
+// whose largest relative error on [0, 1] is smallest (a linear programme over 20001 points; 8.6e-5, far below the bf16
+// rounding of P).  The special-function unit delivers one warp of exponentials per 8 cycles per scheduler; a third of
+// the exponentials go this way so that neither pipe bounds the softmax.
 __device__ __forceinline__ void ex2_poly2(float x0, float x1, float& y0, float& y1) {
   const uint64_t x = pk64(fmaxf(x0, -127.0f), fmaxf(x1, -127.0f));
   const uint64_t magic = pk64(12582912.0f, 12582912.0f), nmagic = pk64(-12582912.0f, -12582912.0f);
@@ -157,8 +158,8 @@ __device__ __forceinline__ void ex2_poly2(float x0, float x1, float& y0, float& 
   const uint64_t fl = add2(t, nmagic);                           // floor(x), exact
   const uint64_t mone = pk64(-1.0f, -1.0f);
   const uint64_t f = fma2(fl, mone, x);                          // x - floor(x), exact
-  uint64_t r = fma2(f, pk64(0.077119089663028717f, 0.077119089663028717f), pk64(0.227564394474029541f, 0.227564394474029541f));
-  r = fma2(r, f, pk64(0.695146143436431885f, 0.695146143436431885f));
+  uint64_t r = fma2(f, pk64(0.0770680314f, 0.0770680314f), pk64(0.227643533f, 0.227643533f));
+  r = fma2(r, f, pk64(0.695117286f, 0.695117286f));
   r = fma2(r, f, pk64(1.0f, 1.0f));
   float r0, r1, t0, t1;
   unpk64(r, r0, r1);
