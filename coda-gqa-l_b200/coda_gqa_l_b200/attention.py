@@ -219,9 +219,9 @@ class CoDAGQALandmarkPerf2(nn.Module):
         # the attention kernel writes the new token itself (coda_b200_decode_attend_append).
         self.fuse_append_into_attention = True
         # chunked prefill: scores and decisions of a block's routing on a second stream beside the block's attention.
-        # Same results; measured slower at the 7B shape (2.27 against 2.15 ms per layer and 512-token chunk: a scoring
-        # CTA and an attention CTA do not fit one SM together, so the scoring kernel takes whole SMs from the attention
-        # for as long as its latency chains last), hence off.
+        # Same results.  Microseconds per prefill without / with it: 64 states of a 512-wide layer (2048 tokens) 1382 /
+        # 1370, 512 of a 576-wide one (256) 1206 / 1198, 32 of a 4096-wide one (512) 1693 / 1738, 8 of an 8192-wide one
+        # (1024) 2708 / 2717: within 1 % to 3 % either way, for a second stream and two events per block, hence off.
         self.overlap_block_routing = False
         # Route the attention / cache-write / routing launches through the torch custom ops (torch.ops.coda_b200.*,
         # see torch_ops.py) instead of the ctypes binding.  Same entry points underneath, so the same bits; states

@@ -180,8 +180,8 @@ void coda_set_error(const char* fmt, ...);
 // ---- chained launches ----------------------------------------------------------------------------
 // The kernels of a prefill block follow one another on a stream, a few microseconds each, and the gap between two
 // launches is one to two.  Launched this way a kernel may be brought onto the SMs while the one before it finishes; it
-// calls grid_chain() before its first global access (writes too), which holds it back until that kernel has
-// completed and lets the next one come.  A 2048-token prefill of 64 states (8 blocks of 5 launches): 1512 -> 1420 us.
+// calls grid_chain() before its first global access (writes too; route_decide, with its reasons at the launch, reads some
+// inputs ahead of it), which holds it back until that kernel has completed and lets the next one come.  A 2048-token prefill of 64 states (8 blocks of 5 launches): 1512 -> 1420 us.
 __device__ __forceinline__ void grid_chain() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

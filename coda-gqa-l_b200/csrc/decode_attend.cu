@@ -1,6 +1,6 @@
 // Fused decode attention for bf16 states (head_dim 64 or 128, up to 8 query heads per KV head).
 //
-// Persistent kernel: one CTA per SM (two at head_dim 64), each walking over (state, KV head) planes plane = blockIdx.x, + gridDim.x, ...
+// Persistent kernel: one CTA per SM (at head_dim 64 two where that is faster, see two_ctas), each walking over (state, KV head) planes plane = blockIdx.x, + gridDim.x, ...
 // The K and V planes of a head -- all W+Me+Ms slots -- are read from HBM exactly once, by TMA
 // (cp.async.bulk.tensor, 128-byte swizzle) into a ring of 64-slot tiles in shared memory.  Three roles:
 //   * one producer warp streams tiles continuously ACROSS plane boundaries, so the ring never drains between

@@ -400,8 +400,8 @@ prefill_attend_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     // The first base is the maximum over the first TWO tiles (128 keys).  A weight at the base is 1 in bf16 and carries
     // no rounding error; where the base lags, the row's largest weight carries up to 2^-8 of itself, and in a row that one
     // key dominates that is the error of the output.  With one tile's maximum the attention of 130 slots and 64
-    // tokens was 2.2e-3 off 64 bits where it now is 2.0e-3, most of it the rounding of the result (queries of twice unit
-    // variance; the rounding of the weights alone: 1.3e-3 against 0.9e-3).
+    // tokens was 2.2e-3 off 64 bits where it now is 2.0e-3, most of it the rounding of the result (queries of standard
+    // deviation 2; the rounding of the weights alone: 1.3e-3 against 0.9e-3).
     // It costs a CTA the wait for the second Q.K^T: 88.4 -> 90.8, 242 -> 254, 90.5 -> 95.5 and 131 -> 137 us at the four shapes above.
     float ahead = -INFINITY;
     if (NT > 1) {

@@ -1,10 +1,12 @@
-// Bank + ring update with one prefill block, as four launches:
-//   route_score   grid (2, B): cosine scores of every candidate against the routing caches as they were
-//                 before the block (a register-tiled fp32 mini-GEMM per bank); per candidate the best
-//                 exact slot/score and the summary argmax go to a small global scratch.
+// Bank + ring update with one prefill block, as four chained launches:
+//   route_score   cosine scores of every candidate against the routing caches as they were before the block (a
+//                 register-tiled fp32 mini-GEMM per bank); per candidate the best exact slot/score and the summary argmax go
+//                 to a small global scratch.  Grid (2, B, Hkv), the heads of a state in one cluster, for 2..8 KV heads;
+//                 (2, B) otherwise.
 //   route_decide  grid (B): the order-dependent decisions (LRU victim ranking, novel-rank assignment,
 //                 stamps, per-slot candidate lists) -> a small per-state plan in global scratch.
-//   route_apply   grid (written slots, B): one CTA per written bank slot: values + cache re-normalisation.
+//   route_apply   values + cache re-normalisation of the written bank slots: a group of one, two or eight warps per slot, by
+//                 the length of its rows; a CTA holds four, two or one group.
 //   ring_rewrite  grid (2*Hkv, B): kept ring rows shift to the front, the block's tail is appended.
 // Semantics: upstream memory_banks.py:438-564 (block write), 633-742 (exact), 853-932 (summary).
 #include "coda_common.cuh"
@@ -883,14 +885,18 @@ static int launch_route(RouteParams& p, cudaStream_t s, int phase = 0) {
                          (size_t)c.Ms + 2) + c.Me + c.Ms + 64;
     CODA_REQUIRE(smem2 <= 200 * 1024, CODA_ERR_LIMIT, "route_block: decision stage needs %zu bytes of shared memory", smem2);
     if (smem2 > 48 * 1024) cudaFuncSetAttribute(route_decide_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    // route_decide reads candidates, gates, slot flags and stamps BEFORE its grid_chain().  That is sound because the launch
+    // just before it on the stream is the scoring kernel above, every CTA of which lets it come only after its own wait (so
+    // whatever wrote these is complete) and which writes ex_best, ex_bi and su_idx only.  No launch may go between the two.
     coda_launch_chained(route_decide_kernel<T>, dim3(c.B), dim3(RD_THREADS), smem2, s, 1, p);
     CODA_CHECK_LAUNCH("route_block (decide)");
   }
   if (phase == 1) return CODA_OK;
   if (p.te > 0 || p.ts > 0) {
     const int tmax = p.te > p.ts ? p.te : p.ts;
+    // The entry point's documented limit.  (The kernel itself needs the new rows only: 4 bytes an element and group.)
     const size_t most = sizeof(float) * (size_t)HD + 8 * (size_t)(tmax > 0 ? tmax : 1);
-    CODA_REQUIRE(most <= 200 * 1024, CODA_ERR_LIMIT, "route_block: Hkv*Dh = %d with %d candidates per block needs %zu bytes of shared memory", HD, tmax, most);
+    CODA_REQUIRE(most <= 200 * 1024, CODA_ERR_LIMIT, "route_block: Hkv*Dh = %d with %d candidates per block exceeds the limit (4 * Hkv*Dh + 8 * candidates = %zu, at most 204800)", HD, tmax, most);
     const int nslots = (c.Me > 0 ? p.te : 0) + (c.Ms > 0 && p.ts > 0 ? c.Ms : 0);
     if (nslots > 0) {
       if constexpr (sizeof(T) == 2) { if (rows_vec16<T>(p)) launch_apply<T, true>(p, nslots, s); else launch_apply<T, false>(p, nslots, s); }
